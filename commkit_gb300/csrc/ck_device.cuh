@@ -30,6 +30,15 @@ constexpr int kPackedDegree = 27;
 __host__ __device__ constexpr int kernel_dmax(bool qc, int max_deg) {
     return max_deg > kPackedDegree ? 0 : (max_deg > 16 ? 27 : ((!qc && max_deg <= 8) ? 8 : 16));
 }
+
+// Codes without circulants (ck_ldpc_ell.cuh): the info byte of a group of 32
+// rows holds its largest degree; kEllSpecial where rows are shorter than that
+// or missing, or touch variables in device memory; and kEllGeneral where more
+// than the last kEllTailEdges edges of a row do so.
+constexpr uint32_t kEllGeneral = 0x80u;
+constexpr uint32_t kEllSpecial = 0x40u;
+constexpr int kEllTailEdges = 2;
+__host__ __device__ constexpr uint32_t ell_degree(uint32_t info) { return info & 0x3fu; }
 }  // namespace ldpc
 
 // q = n / d for 0 <= n < 2^31 and a run-time divisor 1 <= d < 2^31, by a

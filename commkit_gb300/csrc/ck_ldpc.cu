@@ -49,6 +49,7 @@
 #include <utility>
 
 #include "ck_ldpc_cluster.cuh"
+#include "ck_ldpc_ell.cuh"
 #include "ck_ldpc_kernel.cuh"
 #include "ck_ldpc_minsum.cuh"
 #include "ck_ldpc_mixed.cuh"
@@ -68,8 +69,13 @@ template <int DMAX, template <bool> class State>
 struct MinSumPickOf {
     template <bool QC, bool ONE_ROW>
     static KernelFn get(bool app_smem, bool r_smem) {
-        if (app_smem && r_smem) return decode_kernel<State, QC, DMAX, true, true, ONE_ROW>;
-        if (app_smem) return decode_kernel<State, QC, DMAX, true, false, ONE_ROW>;
+        // Codes without circulants and up to kPackedDegree edges per row run
+        // here only where decode_ell_kernel does not take them, which leaves
+        // no posterior small enough for shared memory.
+        if constexpr (QC || DMAX == 0) {
+            if (app_smem && r_smem) return decode_kernel<State, QC, DMAX, true, true, ONE_ROW>;
+            if (app_smem) return decode_kernel<State, QC, DMAX, true, false, ONE_ROW>;
+        }
         if constexpr (!QC) return decode_kernel<State, QC, DMAX, false, false, false>;
         return nullptr;
     }
@@ -86,6 +92,15 @@ struct MinSumPick {
 
 KernelFn min_sum_kernel(bool qc, int max_deg, bool app_smem, bool r_smem, bool one_row) {
     return pick_shape<MinSumPick>(qc, max_deg, app_smem, r_smem, one_row);
+}
+
+KernelFn min_sum_ell_kernel(int max_deg, bool r_smem) {
+    switch (kernel_dmax(false, max_deg)) {
+        case 8: return r_smem ? decode_ell_kernel<MinSumState, 8, true> : decode_ell_kernel<MinSumState, 8, false>;
+        case 16: return r_smem ? decode_ell_kernel<MinSumState, 16, true> : decode_ell_kernel<MinSumState, 16, false>;
+        case 27: return r_smem ? decode_ell_kernel<MinSumState, 27, true> : decode_ell_kernel<MinSumState, 27, false>;
+        default: return nullptr;
+    }
 }
 
 KernelFn min_sum_cluster_kernel(int max_deg) {
@@ -111,6 +126,7 @@ struct Resolved {
     bool app_smem, r_smem;
     uint32_t tables_bytes, group_bytes, gblk_off, app_off, r_off, r_stride, smem;
     int32_t app_stride;
+    size_t app_slot_bytes;  // posterior of one frame slot in device memory (0: all in shared)
     int grid;
     size_t r_slot_bytes;  // message state of one frame slot in device memory (0 in shared)
     size_t ws_bytes, r_ws_off, app_ws_off;
@@ -122,6 +138,7 @@ struct Resolved {
     int plain_grid;  // the plain kernel's grid for the same frames
     int32_t sign_words;  // wide min-sum state: sign words per row (0: packed or sum-product)
     bool edges;  // min-sum with one message per edge in shared memory (CK_LDPC_PLACE_EDGES)
+    bool ell;    // decode_ell_kernel
 };
 
 constexpr int kMaxCluster = 8;  // the portable cluster size
@@ -141,6 +158,15 @@ int device_limits(int dev, int* sms, int* smem_optin) {
 // compiled already (no NVRTC, no module load), and nothing cached.
 int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_sm_out, int* sms_out,
                   bool may_compile);
+
+// Threads per frame of decode_ell_kernel with `frames` frames on an SM: an
+// equal share of the threads its registers allow, no more than the longest
+// layer has rows.
+int32_t ell_threads(const ck_ldpc_plan* plan, int32_t frames) {
+    const int32_t most = ell_max_threads(kernel_dmax(false, plan->max_deg));
+    const int32_t rows = (plan->max_layer_rows + 31) / 32 * 32;
+    return std::max(32, std::min(most / std::max(1, frames) / 32 * 32, rows));
+}
 
 int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool may_compile = true) {
     if (rule != CK_LDPC_MIN_SUM && rule != CK_LDPC_SUM_PRODUCT)
@@ -204,7 +230,15 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
         // same bits.
         const int64_t blocks = int64_t(sms) * per_sm;
         const int32_t g2 = static_cast<int32_t>((B + blocks - 1) / blocks);
-        if (g2 >= 1 && g2 < G) {
+        if (r->ell && plan->launch.threads_per_frame == 0 && plan->launch.frames_per_block == 0) {
+            // One frame per block, its threads the share of an SM that the
+            // frames spread over all SMs leave each (the SMs hold them all:
+            // their shared memory does, and so do those threads).
+            r->T = std::max(r->T, ell_threads(plan, static_cast<int32_t>((B + sms - 1) / sms)));
+            G = r->G = 1;
+            r->smem = r->tables_bytes + r->group_bytes;
+            per_sm = static_cast<int>((B + sms - 1) / sms);
+        } else if (g2 >= 1 && g2 < G) {
             G = g2;
             r->G = g2;
             r->smem = r->tables_bytes + static_cast<uint32_t>(g2) * r->group_bytes;
@@ -222,7 +256,7 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
     r->r_ws_off = kHeaderBytes;
     const size_t r_ws = slots * r->r_slot_bytes;
     r->app_ws_off = kHeaderBytes + ((r_ws + 255) / 256) * 256;
-    const size_t app_ws = r->app_smem ? 0 : slots * static_cast<size_t>(r->app_stride) * 4;
+    const size_t app_ws = slots * r->app_slot_bytes;
     r->ws_bytes = r->app_ws_off + app_ws;
     return CK_OK;
 }
@@ -231,21 +265,23 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
 int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_sm_out, int* sms_out,
                   bool may_compile) {
     const bool sp = rule == CK_LDPC_SUM_PRODUCT;
+    const bool ell = plan->ell && !sp;
     int sms = 0, optin = 0;
     CK_TRY(device_limits(plan->device, &sms, &optin));
     const uint32_t tables =
         plan->qc ? align_up(align_up(static_cast<uint32_t>(plan->L + 1 + plan->mb + 1) * 4, 8) +
                                 static_cast<uint32_t>(plan->nnzb) * 8,
                             128)
-                 : align_up(static_cast<uint32_t>(plan->L + 1) * 4, 128);
+                 : align_up(static_cast<uint32_t>(ell ? 2 * (plan->L + 1) + plan->ell_rows / 32 : plan->L + 1) * 4, 128);
     const uint32_t ctrl = 128;
-    const uint32_t app_bytes = align_up(static_cast<uint32_t>(plan->N) * 4, 128);
+    const uint32_t app_bytes = align_up(static_cast<uint32_t>(ell ? plan->ell_ns + 1 : plan->N) * 4, 128);
     // Message state per frame: min-sum keeps a 16-byte record per row in
     // shared memory (12 bytes in device memory), or for rows above 27 edges
     // the wide state's 3 + sign_words words per row in either; sum-product
     // one float per edge in either.
     const int32_t sign_words = (!sp && plan->max_deg > kPackedDegree) ? (plan->max_deg + 31) / 32 : 0;
-    const uint32_t r_stride = align_up(static_cast<uint32_t>(sp ? plan->E : plan->m), 32);
+    const uint32_t r_stride =
+        align_up(static_cast<uint32_t>(ell ? plan->ell_rows : (sp ? plan->E : plan->m)), 32);
     const uint32_t r_bytes = r_stride * (sp ? 4 : (sign_words ? 4 * (3 + sign_words) : 16));  // in shared memory
     const uint32_t r_bytes_dev = r_stride * (sp ? 4 : (sign_words ? 4 * (3 + sign_words) : 12));  // in device memory
     // Per group: its copy of the circulant table with shared addresses.
@@ -266,7 +302,7 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
             // above 512 threads and still a multiple of 32.
             T = Zp;
             while (T > 512 && T % 64 == 0) T /= 2;
-        } else {
+        } else if (!ell) {  // (ell: below, from the frames that fit)
             const int32_t avg = std::max(1, plan->m / plan->L);
             T = 32;
             while (T < 512 && T < avg / 2) T *= 2;
@@ -277,11 +313,13 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
                         "threads_per_frame %d must divide or be a multiple of %d (the lifting %d "
                         "rounded up to whole warps)",
                         T, Zp, plan->Z);
-    const int32_t max_threads = max_block_threads(plan->qc, kernel_dmax(plan->qc, plan->max_deg));
+    const int32_t dmax = kernel_dmax(plan->qc, plan->max_deg);
+    int32_t max_threads = max_block_threads(plan->qc, dmax);
     if (T > max_threads)
         return ck::fail(CK_ERR_INVALID_ARGUMENT,
                         "threads_per_frame %d above %d for row degree %d", T, max_threads,
                         plan->max_deg);
+    if (ell) max_threads = ell_max_threads(dmax);
 
     bool r_smem;
     uint32_t r_used = r_bytes, r_stride_used = r_stride;
@@ -321,6 +359,8 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
         r_smem = 2 * (ctrl + gblk_bytes + app_bytes + r_bytes) <= budget;
     }
     uint32_t group = ctrl + gblk_bytes + (app_smem ? app_bytes : 0) + (r_smem ? r_used : 0);
+    if (ell)
+        T = T ? std::min(T, max_threads) : ell_threads(plan, static_cast<int32_t>(budget / group));
     int32_t G = sp ? 0 : plan->launch.frames_per_block;
     const int32_t gmax_threads = max_threads / T;
     const int32_t gmax_smem = static_cast<int32_t>(budget / group);
@@ -329,9 +369,20 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
     if (gmax < 1)
         return ck::fail(CK_ERR_UNSUPPORTED, "a frame needs %u bytes of shared memory, %u available",
                         group, budget);
+    if (ell && G > gmax) {
+        // A set shape is cut to what this kernel's blocks hold, unless the
+        // threads, barriers or whole frames in shared memory of any kernel of
+        // the code would refuse it.
+        const uint32_t whole = ctrl + align_up(static_cast<uint32_t>(plan->N) * 4, 128) + (r_smem ? r_used : 0);
+        const int32_t any = std::min(max_block_threads(false, dmax) / T, gmax_bar);
+        if (G <= any && (plan->ell_ns < plan->N || G <= static_cast<int32_t>(static_cast<uint32_t>(optin) / whole)))
+            G = gmax;
+    }
     const bool one_row = plan->qc && T >= Zp;
-    const KernelFn table = sp ? sum_product_kernel(plan->qc, plan->max_deg, app_smem, r_smem, one_row)
-                              : min_sum_kernel(plan->qc, plan->max_deg, app_smem, r_smem, one_row);
+    const KernelFn table =
+        ell ? min_sum_ell_kernel(plan->max_deg, r_smem)
+            : (sp ? sum_product_kernel(plan->qc, plan->max_deg, app_smem, r_smem, one_row)
+                  : min_sum_kernel(plan->qc, plan->max_deg, app_smem, r_smem, one_row));
     if (!table) return ck::fail(CK_ERR_UNSUPPORTED, "no decoder kernel for this code shape");
     const void* kernel = reinterpret_cast<const void*>(table);
     if (edge_kernel) {
@@ -381,7 +432,9 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
     r->r_stride = r_stride_used;
     r->edges = edge_kernel != nullptr;
     r->smem = tables + static_cast<uint32_t>(G) * group;
-    r->app_stride = static_cast<int32_t>(app_bytes / 4);
+    r->app_stride = static_cast<int32_t>(ell ? align_up(static_cast<uint32_t>(plan->N - plan->ell_ns), 32)
+                                             : app_bytes / 4);
+    r->app_slot_bytes = ell || !app_smem ? static_cast<size_t>(r->app_stride) * 4 : 0;
     r->sign_words = sign_words;
 
     int per_sm = 0;
@@ -395,7 +448,8 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
     r->cluster_kernel = nullptr;
     r->cluster_per_sm = 0;
     r->cluster = 1;
-    if (!plan->qc && !app_smem && !r_smem) {
+    r->ell = ell;
+    if (!plan->qc && !ell && !app_smem && !r_smem) {
         KernelFn ck = sp ? sum_product_cluster_kernel(plan->max_deg) : min_sum_cluster_kernel(plan->max_deg);
         int cps = 0;
         CK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cps, reinterpret_cast<const void*>(ck), T, 0));
@@ -507,7 +561,7 @@ Params make_params(const ck_ldpc_plan* plan, const Resolved& r, const float* llr
     p.divZ = plan->divZ;
     p.Zp = plan->qc ? (plan->Z + 31) / 32 * 32 : 32;
     p.q_bstep = (plan->qc && r.T >= p.Zp) ? r.T / p.Zp : 1;
-    p.layer = plan->d_layer;
+    p.layer = r.ell ? plan->d_ell_layer : plan->d_layer;
     p.eptr = plan->d_eptr;
     p.blk = reinterpret_cast<const int2*>(plan->d_blk);
     p.cols = plan->d_cols;
@@ -533,6 +587,11 @@ Params make_params(const ck_ldpc_plan* plan, const Resolved& r, const float* llr
     p.g_app = reinterpret_cast<float*>(wsb + r.app_ws_off);
     p.app_stride = r.app_stride;
     p.sign_words = r.sign_words;
+    p.ell = reinterpret_cast<const uint4*>(plan->d_ell_cols);
+    p.ell_info = reinterpret_cast<const uint32_t*>(plan->d_ell_info);
+    p.ell_rows = static_cast<uint32_t>(plan->ell_rows);
+    p.ell_ns = plan->ell_ns;
+    if (r.ell) p.m = plan->ell_rows;
     return p;
 }
 
@@ -625,7 +684,7 @@ int ck::ldpc_decode_in_scratch(const ck_ldpc_plan* plan, const float* llr_in, fl
     r.cluster = 1;
     r.grid = r.plain_grid;
     // Bytes of device-memory state per frame slot (the header is shared).
-    const size_t app_bytes = r.app_smem ? 0 : static_cast<size_t>(r.app_stride) * 4;
+    const size_t app_bytes = r.app_slot_bytes;
     const size_t per_slot = r.r_slot_bytes + app_bytes;
     if (per_slot > 0) {
         const size_t usable = scratch_bytes > kHeaderBytes + 256 ? scratch_bytes - kHeaderBytes - 256 : 0;

@@ -49,6 +49,17 @@ struct ck_ldpc_plan {
     int32_t* d_eptr = nullptr;
     int32_t* d_blk = nullptr;
     int32_t* d_cols = nullptr;
+    // Form of codes without circulants, up to kPackedDegree edges per row and
+    // 65,535 variables, for min-sum (decode_ell_kernel): rows renumbered per
+    // layer (ell_layer: first row and end of each, the first a multiple of
+    // 32; ell_rows in all), their 16-bit columns and a word per 32 rows;
+    // variables [0, ell_ns) in shared memory.
+    bool ell = false;
+    int32_t ell_rows = 0, ell_ns = 0;
+    std::vector<int32_t> ell_layer, ell_cols, ell_info;
+    int32_t* d_ell_layer = nullptr;
+    int32_t* d_ell_cols = nullptr;
+    int32_t* d_ell_info = nullptr;
     ck::FastDiv divZ{1, 1, 0};
     ck_ldpc_launch launch{0, 0, 0};
     // The decoder's launch shape per check rule for the current launch
@@ -59,7 +70,7 @@ struct ck_ldpc_plan {
         ck_ldpc_launch launch{0, 0, 0};
         int32_t jit_mode = 0;
         int per_sm = 0, sms = 0;
-        alignas(16) unsigned char resolved[192];
+        alignas(16) unsigned char resolved[224];
     };
     mutable ShapeCache shape_cache[2];
     mutable std::mutex shape_mu;

@@ -67,6 +67,14 @@ struct Params {
     // Min-sum codes with rows above kPackedDegree edges: sign words per row
     // of the wide message state (0 otherwise).
     int32_t sign_words;
+    // Codes decoded by decode_ell_kernel (ck_ldpc_ell.cuh): layer holds the
+    // first row and end of each layer in its numbering (ell_rows rows), ell 8
+    // 16-bit columns per entry (entry c ell_rows + row), ell_info a word per
+    // 32 rows; variables [0, ell_ns) in shared memory, the rest in g_app.
+    const uint4* ell;
+    const uint32_t* ell_info;
+    uint32_t ell_rows;
+    int32_t ell_ns;
 };
 
 __device__ __forceinline__ float flip_sign(float v, uint32_t bit) {
@@ -208,7 +216,7 @@ template <class ColOf>
 struct CsrPost {
     float* a;
     const ColOf& col_of;
-    __device__ __forceinline__ uint32_t col(uint32_t e) const { return static_cast<uint32_t>(col_of(static_cast<int>(e))); }
+    __device__ __forceinline__ uint32_t col(int e) const { return static_cast<uint32_t>(col_of(e)); }
     __device__ __forceinline__ float ld(uint32_t c) const { return a[c]; }
     __device__ __forceinline__ void st(uint32_t c, float v) const { a[c] = v; }
 };

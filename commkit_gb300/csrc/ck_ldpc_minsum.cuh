@@ -4,39 +4,37 @@
 // kernels compiled at run time (ck_ldpc_jit.cu).  Compiles under NVRTC.
 #pragma once
 
-#include "ck_ldpc_kernel.cuh"
+#include "ck_ldpc_ell.cuh"
 
 namespace ck {
 namespace ldpc {
 
-
 // One check row, min-sum: reads the row's compressed state (m1, m2, w),
-// updates the posterior `a` of its deg variables (columns from col_of) and
+// updates the posterior of its deg variables (handles post.col(e)) and
 // writes the new state back.  Two passes as the reference's min_sum_row
 // (commkit/_cuda/src/ldpc.cu:45-72), with Q and the columns kept in
 // registers between them.
-template <int DMAX, class ColOf>
-__device__ __forceinline__ void min_sum_row(float* __restrict__ a, const int deg,
-                                            const ColOf& col_of, float& m1, float& m2,
+template <int DMAX, class Post>
+__device__ __forceinline__ void min_sum_row(const Post& post, const int deg, float& m1, float& m2,
                                             uint32_t& w, const float scale,
                                             const float offset) {
     const uint32_t oidx = w >> 27;
     const uint32_t osign = w;
     const float om1 = m1, om2 = m2;
     float q[DMAX];
-    int col[DMAX];  // loaded once, all before the first posterior load
+    uint32_t col[DMAX];  // loaded once, all before the first posterior load
     float min1 = ck::inf_f(), min2 = ck::inf_f();
     uint32_t idx = 31u;  // no edge; matches the reference's -1 when every |Q| is inf
     uint32_t negs = 0u;
 #pragma unroll
     for (int e = 0; e < DMAX; ++e)
-        if (e < deg) col[e] = col_of(e);
+        if (e < deg) col[e] = post.col(e);
 #pragma unroll
     for (int e = 0; e < DMAX; ++e) {
         if (e < deg) {
             const float r_old =
                 flip_sign(static_cast<uint32_t>(e) == oidx ? om2 : om1, (osign >> e) & 1u);
-            const float qe = __fsub_rn(a[col[e]], r_old);
+            const float qe = __fsub_rn(post.ld(col[e]), r_old);
             q[e] = qe;
             negs |= (qe < 0.0f ? 1u : 0u) << e;
             const float mag = fabsf(qe);
@@ -53,7 +51,7 @@ __device__ __forceinline__ void min_sum_row(float* __restrict__ a, const int deg
     for (int e = 0; e < DMAX; ++e) {
         if (e < deg) {
             const float rn = flip_sign(static_cast<uint32_t>(e) == idx ? n2 : n1, (signs >> e) & 1u);
-            a[col[e]] = __fadd_rn(q[e], rn);
+            post.st(col[e], __fadd_rn(q[e], rn));
         }
     }
     m1 = n1;
@@ -79,10 +77,15 @@ __device__ __forceinline__ void min_sum_row(float* __restrict__ a, const int deg
 //    means min2 == min1, so every tied edge gets the same value), and the
 //    stored argmin is the first such edge, found in the second pass.
 // The compressed state keeps the sign of edge e at bit D - 1 - e here.
-// The row's columns come as shared-memory addresses c[0..D).
-template <int D>
+// The row's columns come as handles c[0..D) of `mem` (SmemRow: shared-memory
+// addresses).
+struct SmemRow {
+    __device__ __forceinline__ float ld(int, uint32_t c) const { return ld_shared_f32(c); }
+    __device__ __forceinline__ void st(int, uint32_t c, float v) const { st_shared_f32(c, v); }
+};
+template <int D, class Mem = SmemRow>
 __device__ __forceinline__ void qc_row_cols(const uint32_t (&c)[D], float& m1, float& m2, uint32_t& w,
-                                            const float scale, const float offset) {
+                                            const float scale, const float offset, const Mem& mem = Mem()) {
     const uint32_t oidx = w >> 27;
     const uint32_t osign = w;
     const float om1 = m1, om2 = m2;
@@ -95,7 +98,7 @@ __device__ __forceinline__ void qc_row_cols(const uint32_t (&c)[D], float& m1, f
         const float mag_old = static_cast<uint32_t>(e) == oidx ? om2 : om1;
         const float r_old = __uint_as_float(__float_as_uint(mag_old) ^
                                             ((osign << (32 - D + e)) & 0x80000000u));
-        const float qe = __fsub_rn(ld_shared_f32(ce), r_old);
+        const float qe = __fsub_rn(mem.ld(e, ce), r_old);
         q[e] = qe;
         negs = __funnelshift_l(__float_as_uint(qe), negs, 1);
         if (e & 1) {
@@ -127,7 +130,7 @@ __device__ __forceinline__ void qc_row_cols(const uint32_t (&c)[D], float& m1, f
         const float mag = at_min ? n2 : n1;
         const float t = __fmul_rn(q[e], psign);
         const float rn = __uint_as_float(__float_as_uint(mag) | (__float_as_uint(t) & 0x80000000u));
-        st_shared_f32(c[e], __fadd_rn(q[e], rn));
+        mem.st(e, c[e], __fadd_rn(q[e], rn));
     }
     const uint32_t signs = negs ^ (odd ? ((1u << D) - 1u) : 0u);
     m1 = n1;
@@ -200,6 +203,62 @@ __device__ __forceinline__ void qc_row(const int2* __restrict__ gblk, const int 
     }
 }
 #undef CK_ROW_CASE
+
+// The same row body at the 16-bit places of a 32-row group of largest degree
+// D: every column a variable in shared memory, or (special groups) also the
+// +inf word of a missing edge, whose store is left out, and in the last
+// kEllTailEdges edges a variable in device memory, whose load goes out
+// before all others.
+template <int D>
+struct EllSpecialRow {
+    float t[kEllTailEdges];
+    float* g;      // the place after the +inf word
+    uint32_t inf;  // the +inf word's shared address
+    template <class Post>
+    __device__ __forceinline__ EllSpecialRow(const Post& post, const uint32_t (&c)[D])
+        : g(post.g), inf(post.a_addr + 4u * post.ns) {
+#pragma unroll
+        for (int i = 0; i < kEllTailEdges; ++i) {
+            const int e = D - kEllTailEdges + i;
+            t[i] = 0.0f;
+            if (e >= 0 && c[e] > inf) t[i] = __ldcg(at(c[e]));
+        }
+    }
+    __device__ __forceinline__ float* at(uint32_t c) const {
+        return reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(g) + (c - inf - 4u));
+    }
+    __device__ __forceinline__ float ld(int e, uint32_t c) const {
+        if (e >= D - kEllTailEdges && c > inf) return t[e - (D - kEllTailEdges)];
+        return ld_shared_f32(c);
+    }
+    __device__ __forceinline__ void st(int e, uint32_t c, float v) const {
+        if (c < inf)
+            st_shared_f32(c, v);
+        else if (e >= D - kEllTailEdges && c > inf)
+            __stcg(at(c), v);
+    }
+};
+template <int D, class Post>
+__device__ __forceinline__ void ell_row_fixed(const Post& post, const bool special, float& m1, float& m2,
+                                              uint32_t& w, const float scale, const float offset) {
+    uint32_t c[D];
+#pragma unroll
+    for (int e = 0; e < D; ++e) c[e] = post.a_addr + 4u * post.col(e);
+    if (special)
+        qc_row_cols<D>(c, m1, m2, w, scale, offset, EllSpecialRow<D>(post, c));
+    else
+        qc_row_cols<D>(c, m1, m2, w, scale, offset);
+}
+template <int D, class Post>
+__device__ __forceinline__ void ell_row_degree(const int deg, const Post& post, const bool special, float& m1,
+                                               float& m2, uint32_t& w, const float scale, const float offset) {
+    if constexpr (D >= 2) {
+        if (deg == D)
+            ell_row_fixed<D>(post, special, m1, m2, w, scale, offset);
+        else
+            ell_row_degree<D - 1>(deg, post, special, m1, m2, w, scale, offset);
+    }
+}
 
 // Min-sum check-message state of a frame slot: per row (min1', min2', one
 // word of signs and argmin).  In shared memory one 16-byte record per row
@@ -315,7 +374,22 @@ struct MinSumState {
         const uint4 s = load(row);
         float m1 = __uint_as_float(s.x), m2 = __uint_as_float(s.y);
         uint32_t w = s.z;
-        min_sum_row<DMAX>(a, deg, col_of, m1, m2, w, p.scale, p.offset);
+        min_sum_row<DMAX>(CsrPost<ColOf>{a, col_of}, deg, m1, m2, w, p.scale, p.offset);
+        store(row, m1, m2, w);
+    }
+    // One row of a code without circulants (decode_ell_kernel): the row body
+    // of its group's largest degree, or the general one (each row always
+    // takes the same, so the two layouts of the sign bits never meet).
+    template <int DMAX, int W>
+    __device__ __forceinline__ void ell_row(const Params& p, const EllRow<W>& r, const EllPost<W>& post,
+                                            uint32_t row) const {
+        const int deg = static_cast<int>(ell_degree(r.info));
+        float m1 = __uint_as_float(r.state.x), m2 = __uint_as_float(r.state.y);
+        uint32_t w = r.state.z;
+        if (r.info & kEllGeneral)
+            min_sum_row<DMAX>(post, deg, m1, m2, w, p.scale, p.offset);
+        else
+            ell_row_degree<DMAX>(deg, post, (r.info & kEllSpecial) != 0u, m1, m2, w, p.scale, p.offset);
         store(row, m1, m2, w);
     }
 };

@@ -152,6 +152,122 @@ bool try_qc(const int32_t* row_ptr, const int32_t* cols, const int32_t* layer_pt
     return true;
 }
 
+// Rows of one layer and degree in an order that spreads the lanes of each
+// shared-memory access over the banks: groups of 32 are filled row by row,
+// each time with the row of the next kWindow that raises the groups' largest
+// bank counts least (then the one meeting the fewest taken banks), the first
+// among equals.  cols(r)[e] is edge e's variable.
+template <class Cols>
+void spread_banks(std::vector<int32_t>& rows, int32_t deg, const Cols& cols) {
+    constexpr size_t kWindow = 128;
+    std::vector<int32_t> window, out;
+    out.reserve(rows.size());
+    size_t next = 0;
+    std::vector<uint8_t> count(static_cast<size_t>(deg) * 32), top(static_cast<size_t>(deg));
+    while (out.size() < rows.size()) {
+        if (out.size() % 32 == 0) {
+            std::fill(count.begin(), count.end(), 0);
+            std::fill(top.begin(), top.end(), 0);
+        }
+        while (window.size() < kWindow && next < rows.size()) window.push_back(rows[next++]);
+        size_t best = 0;
+        int32_t best_cost = INT32_MAX;
+        for (size_t i = 0; i < window.size() && best_cost > 0; ++i) {
+            const int32_t* c = cols(window[i]);
+            int32_t cost = 0;
+            for (int32_t e = 0; e < deg && cost < best_cost; ++e) {
+                const int32_t n = count[static_cast<size_t>(e) * 32 + (c[e] & 31)];
+                cost += n + (n >= top[e] ? 1024 : 0);
+            }
+            cost -= 1024 * (out.size() % 32 == 0 ? deg : 0);  // a group's first row raises every count
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = i;
+            }
+        }
+        const int32_t r = window[best];
+        window.erase(window.begin() + static_cast<int64_t>(best));
+        const int32_t* c = cols(r);
+        for (int32_t e = 0; e < deg; ++e) {
+            const uint8_t n = ++count[static_cast<size_t>(e) * 32 + (c[e] & 31)];
+            top[e] = std::max(top[e], n);
+        }
+        out.push_back(r);
+    }
+    rows.swap(out);
+}
+
+// The ELL form of a code without circulants (ck_ldpc_ell.cuh), when it has
+// one: `smem` bytes of shared memory per block.
+void make_ell(const int32_t* row_ptr, const int32_t* cols, const int32_t* layer_ptr, int32_t smem,
+              ck_ldpc_plan* plan) {
+    const int32_t L = plan->L, N = plan->N;
+    if (plan->max_deg > ck::ldpc::kPackedDegree || N > 65535) return;  // places up to N in 16 bits
+    // First row and end of each layer, then an empty one.
+    std::vector<int32_t>& range = plan->ell_layer;
+    range.clear();
+    int32_t rows = 0;
+    for (int32_t l = 0; l < L; ++l) {
+        const int32_t count = layer_ptr[l + 1] - layer_ptr[l];
+        range.push_back(rows);
+        range.push_back(rows + count);
+        rows += (count + 31) / 32 * 32;
+    }
+    range.push_back(0);
+    range.push_back(0);
+    plan->ell_rows = rows;
+    // Variables in shared memory: what the tables, a control block and the
+    // +inf word leave.
+    const int64_t room =
+        static_cast<int64_t>(smem) - (static_cast<int64_t>(2 * (L + 1) + rows / 32) * 4 + 127) / 128 * 128 - 128;
+    const int64_t fit = room / 128 * 32 - 32;
+    if (fit < N / 2) return;
+    const int32_t ns = plan->ell_ns = static_cast<int32_t>(std::min<int64_t>(N, fit));
+    plan->ell = true;
+    const int32_t chunks = (plan->max_deg + 7) / 8;
+    std::vector<uint16_t> c16(static_cast<size_t>(chunks) * rows * 8, static_cast<uint16_t>(ns));
+    plan->ell_info.assign(static_cast<size_t>(rows) / 32, 0);
+    const auto deg_of = [&](int32_t r) { return row_ptr[r + 1] - row_ptr[r]; };
+    const auto cols_of = [&](int32_t r) { return cols + row_ptr[r]; };
+    std::vector<int32_t> order;
+    std::vector<std::vector<int32_t>> by_deg, tail_by_deg;
+    for (int32_t l = 0; l < L; ++l) {
+        order.clear();
+        by_deg.assign(static_cast<size_t>(plan->max_deg) + 1, {});
+        tail_by_deg = by_deg;
+        for (int32_t r = layer_ptr[l]; r < layer_ptr[l + 1]; ++r)  // columns increase along a row: the last one decides
+            (cols[row_ptr[r + 1] - 1] >= ns ? tail_by_deg : by_deg)[deg_of(r)].push_back(r);
+        for (int32_t d = plan->max_deg; d >= 2; --d)
+            order.insert(order.end(), tail_by_deg[d].begin(), tail_by_deg[d].end());
+        for (int32_t d = plan->max_deg; d >= 2; --d) {
+            spread_banks(by_deg[d], d, cols_of);
+            order.insert(order.end(), by_deg[d].begin(), by_deg[d].end());
+        }
+        for (size_t g = 0; g < order.size(); g += 32) {
+            const size_t at0 = static_cast<size_t>(range[2 * l]) + g;
+            const size_t count = std::min<size_t>(32, order.size() - g);
+            int32_t top = 0;
+            for (size_t i = 0; i < count; ++i) top = std::max(top, deg_of(order[g + i]));
+            bool general = false, special = count < 32;
+            for (size_t i = 0; i < count; ++i) {
+                const int32_t r = order[g + i], d = deg_of(r);
+                special |= d != top || cols_of(r)[d - 1] >= ns;
+                for (int32_t e = 0; e < d; ++e) {
+                    const int32_t c = cols_of(r)[e];
+                    general |= c >= ns && e < top - ck::ldpc::kEllTailEdges;
+                    c16[(static_cast<size_t>(e / 8) * rows + at0 + i) * 8 + e % 8] =
+                        static_cast<uint16_t>(c >= ns ? c + 1 : c);
+                }
+            }
+            plan->ell_info[at0 / 32] =
+                static_cast<int32_t>(static_cast<uint32_t>(top) | (general ? ck::ldpc::kEllGeneral : 0u) |
+                                     (special ? ck::ldpc::kEllSpecial : 0u));
+        }
+    }
+    plan->ell_cols.resize(c16.size() / 2);
+    memcpy(plan->ell_cols.data(), c16.data(), c16.size() * 2);
+}
+
 int upload(const std::vector<int32_t>& h, int32_t** d) {
     *d = nullptr;
     if (h.empty()) return CK_OK;
@@ -254,9 +370,18 @@ extern "C" int ck_ldpc_plan_create(const int32_t* row_ptr, const int32_t* cols,
         if (status == CK_OK) status = upload(plan->h_eptr, &plan->d_eptr);
         if (status == CK_OK) status = upload(plan->h_blk, &plan->d_blk);
     } else {
+        int smem = 0;
+        status = ck::cuda_check(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, plan->device),
+                                "cudaDeviceGetAttribute");
+        if (status == CK_OK) make_ell(row_ptr, cols, layer_ptr, smem, plan);
         plan->h_layer.assign(layer_ptr, layer_ptr + L + 1);
+        if (status == CK_OK && plan->ell) {
+            status = upload(plan->ell_layer, &plan->d_ell_layer);
+            if (status == CK_OK) status = upload(plan->ell_cols, &plan->d_ell_cols);
+            if (status == CK_OK) status = upload(plan->ell_info, &plan->d_ell_info);
+        }
         std::vector<int32_t> rp(row_ptr, row_ptr + m + 1), cc(cols, cols + plan->E);
-        status = upload(plan->h_layer, &plan->d_layer);
+        if (status == CK_OK) status = upload(plan->h_layer, &plan->d_layer);
         if (status == CK_OK) status = upload(rp, &plan->d_eptr);
         if (status == CK_OK) status = upload(cc, &plan->d_cols);
     }
@@ -306,6 +431,9 @@ extern "C" int ck_ldpc_plan_destroy(ck_ldpc_plan* plan) {
     if (plan->d_eptr) (void)cudaFree(plan->d_eptr);
     if (plan->d_blk) (void)cudaFree(plan->d_blk);
     if (plan->d_cols) (void)cudaFree(plan->d_cols);
+    if (plan->d_ell_layer) (void)cudaFree(plan->d_ell_layer);
+    if (plan->d_ell_cols) (void)cudaFree(plan->d_ell_cols);
+    if (plan->d_ell_info) (void)cudaFree(plan->d_ell_info);
     ck::ldpc::forget_plan_kernels(plan);
     if (dev >= 0 && dev != plan->device) (void)cudaSetDevice(dev);
     delete plan;
