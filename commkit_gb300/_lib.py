@@ -55,6 +55,7 @@ EXPORTS = (
     "ck_llr_points_frames",
     "ck_random_bits",
     "ck_ldpc_encode",
+    "ck_ldpc_encode_checked",
     "ck_ldpc_encode_generator",
     "ck_ldpc_column_signs",
     "ck_map_awgn",
@@ -203,6 +204,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "ck_llr_points_frames": ([p, i64, i64, p, p, p, p, i32, i32, i32, p, p], ctypes.c_int),
         "ck_random_bits": ([p, i64, ctypes.c_uint64, ctypes.c_uint64, p], ctypes.c_int),
         "ck_ldpc_encode": ([p, i64, i32, i32, i32, p, p, i32, p, p, ctypes.c_size_t, p, p], ctypes.c_int),
+        "ck_ldpc_encode_checked": ([p, i64, i32, i32, i32, p, p, i32, p, p, p], ctypes.c_int),
         "ck_ldpc_encode_generator": ([p, i64, i32, i32, i32, p, p, p, p, ctypes.c_size_t, p, p], ctypes.c_int),
         "ck_ldpc_column_signs": ([p, i64, i32, p, i32, p, p], ctypes.c_int),
         "ck_map_awgn": ([p, i64, i32, p, ctypes.c_float, ctypes.c_float, ctypes.c_uint64, ctypes.c_uint64, p, p],

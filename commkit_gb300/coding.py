@@ -805,6 +805,36 @@ def encode_blocks(code: LDPCCode, info: Any, words: Any = None, scratch: Any = N
     return words
 
 
+def _encode_checked(bits: Any, x: _device.DeviceArray, code: LDPCCode) -> Any:
+    """:func:`encode` of int8 or uint8 torch bits by an accumulator: one
+    kernel reads the bits, checks them and writes the codewords (the checks
+    as passes of their own took as long as the encoding).  None where it does
+    not apply: other types, encoders and shapes, no bits, or information
+    bits that exceed the kernel's shared memory."""
+    if x.kind != "torch" or x.dtype.kind not in "iu" or x.dtype.itemsize != 1 or x.ndim not in (1, 2) or x.size == 0:
+        return None
+    e = code._encoder
+    k, n = code.k, code.n
+    if e.inverse is not None or e.generator is not None or x.shape[-1] % k:
+        return None
+    import torch
+
+    t = bits.contiguous().view(torch.int8)
+    R = t.numel() // k
+    words = torch.empty((*t.shape[:-1], t.shape[-1] // k * n), dtype=torch.int8, device=t.device)
+    bad = torch.zeros(1, dtype=torch.int32, device=t.device)
+    with _device.on_device(x):
+        rp, ci, _ = _encoder_tables(code, x)
+        st = _lib.lib().ck_ldpc_encode_checked(t.data_ptr(), R, k, code.num_checks, n, rp.data_ptr(), ci.data_ptr(),
+                                               e.stride, words.data_ptr(), bad.data_ptr(), _device.stream_of(x))  # fmt: skip
+    if st == _lib.CK_ERR_UNSUPPORTED:
+        return None
+    _lib.check(st, "encode()")
+    if bad.item():
+        raise ValueError("encode(): bits must be 0 or 1.")
+    return words
+
+
 def encode(bits: Any, *, code: LDPCCode) -> Any:
     """Encode information bits (``commkit/coding/base.py:248-290``).
 
@@ -819,6 +849,9 @@ def encode(bits: Any, *, code: LDPCCode) -> Any:
     x = _device.wrap(bits, "bits")
     if x.dtype.kind not in "biu":
         raise TypeError(f"encode(): bits must be integers or bool, got {x.dtype}.")
+    out = _encode_checked(bits, x, code)
+    if out is not None:
+        return out
     t = bits
     if x.kind == "torch":
         import torch

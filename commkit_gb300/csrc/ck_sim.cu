@@ -15,11 +15,15 @@
 // same in every launch shape and on the host (tests restate it in NumPy).
 // Gaussian noise is Box-Muller on two uniforms in (0, 1).
 //
-// Every kernel is a plain grid over its outputs with bounds checks; the
-// encoder's long accumulator chains use one block-wide XOR scan per chain.
+// Every kernel is a plain grid over its outputs with bounds checks.  The
+// accumulator encoder is ck_ldpc_encode.cu; the encoding kernels here serve a
+// GF(2) inverse, a systematic generator, and accumulators whose information
+// bits exceed a block's shared memory (long chains by one block-wide XOR scan
+// per chain).
 #include <stdint.h>
 
 #include "ck_common.cuh"
+#include "ck_ldpc_encode.h"
 
 namespace {
 
@@ -401,6 +405,13 @@ extern "C" int ck_ldpc_encode(const int8_t* info, int64_t B, int32_t k, int32_t 
     if (scratch_bytes < need)
         return ck::fail(CK_ERR_INVALID_ARGUMENT, "scratch of %zu bytes, %zu needed", scratch_bytes, need);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!inverse) {
+        bool done = false;
+        CK_TRY(ck::encode_accumulate(info, B, k, m, n, info_row_ptr, info_cols, stride, words, nullptr, st, &done));
+        if (done) return CK_OK;
+    }
+    // A GF(2) inverse, or an accumulator whose information bits exceed a
+    // block's shared memory.
     copy_info_kernel<<<grid_for(static_cast<uint64_t>(B) * k), kThreads, 0, st>>>(info, B, k, n, words);
     syndrome_kernel<<<grid_for(static_cast<uint64_t>(B) * m), kThreads, 0, st>>>(info, B, k, m, info_row_ptr,
                                                                                   info_cols, scratch);
@@ -422,6 +433,24 @@ extern "C" int ck_ldpc_encode(const int8_t* info, int64_t B, int32_t k, int32_t 
                                                                                    words);
     }
     return ck::cuda_check(cudaGetLastError(), "encoder launch");
+}
+
+extern "C" int ck_ldpc_encode_checked(const int8_t* info, int64_t B, int32_t k, int32_t m, int32_t n,
+                                      const int32_t* info_row_ptr, const int32_t* info_cols, int32_t stride,
+                                      int8_t* words, int32_t* bad, void* stream) {
+    ck::clear_error();
+    if (B < 0 || k < 1 || m < 1 || n < k || n > k + m || stride < 1)
+        return ck::fail(CK_ERR_INVALID_ARGUMENT, "bad sizes (B=%lld k=%d m=%d n=%d stride=%d)",
+                        static_cast<long long>(B), k, m, n, stride);
+    if (B == 0) return CK_OK;
+    if (!info || !words || !info_row_ptr || !info_cols || !bad)
+        return ck::fail(CK_ERR_INVALID_ARGUMENT, "an array is NULL");
+    bool done = false;
+    CK_TRY(ck::encode_accumulate(info, B, k, m, n, info_row_ptr, info_cols, stride, words, bad,
+                                 static_cast<cudaStream_t>(stream), &done));
+    if (!done)
+        return ck::fail(CK_ERR_UNSUPPORTED, "%d information bits exceed a block's shared memory", k);
+    return CK_OK;
 }
 
 extern "C" int ck_ldpc_encode_generator(const int8_t* info, int64_t B, int32_t k, int32_t rank, int32_t n,

@@ -174,6 +174,17 @@ int ck_ldpc_encode(const int8_t* info, int64_t B, int32_t k, int32_t m, int32_t 
                    void* stream);
 
 /*
+ * The accumulator form without scratch, checking the information bits as it
+ * reads them: *bad (device memory) is set to 1 when a byte is not 0 or 1 and
+ * otherwise left as it is; words are then [info | parity of the bytes' low
+ * bits].  CK_ERR_UNSUPPORTED, with nothing launched, when the k information
+ * bits of a group of frames (4 bytes each) exceed a block's shared memory.
+ */
+int ck_ldpc_encode_checked(const int8_t* info, int64_t B, int32_t k, int32_t m, int32_t n,
+                           const int32_t* info_row_ptr, const int32_t* info_cols, int32_t stride, int8_t* words,
+                           int32_t* bad, void* stream);
+
+/*
  * Encoding through a systematic generator, for parity-check matrices whose
  * last m columns are not invertible (the reference's "dense" kind,
  * commkit/coding/ldpc.py:476-481 and :511-533): information bit j goes to
