@@ -26,8 +26,8 @@
 //    chunk (2.6 per point instead of 5 predicated ones per point and bit),
 //    and the chunk's maximum goes to the halves of the higher bits.  Max
 //    is exact and order-free, so this is bit-identical to the reference's
-//    per-point loop.  (Two symbols per thread with two-lane metrics ran no
-//    faster here: 221 against 188 us for 128-cross-QAM.)
+//    per-point loop.  Points of one prior (every constellation without
+//    shaping) go two symbols at a time by distance (nearest_tree).
 //  * The exact method from a staged table whose labels are the points' own
 //    order (every factory-built constellation) takes each symbol's peak
 //    metric, then adds exp(m - peak) to each bit's half point by point, in
@@ -48,6 +48,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "ck_llr_cross.cuh"
 #include "ck_llr_kernels.cuh"
 
 namespace ck {
@@ -135,6 +136,95 @@ __device__ __forceinline__ void maxima_tree(const float4* __restrict__ tab, floa
                 p1[K - 1 - q] = fmaxf(p1[K - 1 - q], a[0]);
             else
                 p0[K - 1 - q] = fmaxf(p0[K - 1 - q], a[0]);
+        }
+    }
+}
+
+// Smallest of three; a NaN counts as absent.
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// One level of the chunk min-tree (tree_level on distances, three inputs to
+// an operation): both halves of bit r, then the fold.  LAST: the fold of bit
+// 0, the chunk's minimum, is wanted too.
+template <int K, int r, bool LAST>
+__device__ __forceinline__ void near_level(float* a, float* p0, float* p1) {
+    if constexpr (r >= 0) {
+        constexpr int h = 1 << r;
+        float lo = p0[K - 1 - r], hi = p1[K - 1 - r];
+        if constexpr (h == 1) {
+            lo = fminf(lo, a[0]);
+            hi = fminf(hi, a[1]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < h; j += 2) {
+                lo = min3(lo, a[j], a[j + 1]);
+                hi = min3(hi, a[h + j], a[h + j + 1]);
+            }
+        }
+        p0[K - 1 - r] = lo;
+        p1[K - 1 - r] = hi;
+        if constexpr (r > 0 || LAST) {
+#pragma unroll
+            for (int j = 0; j < h; ++j) a[j] = fminf(a[j], a[j + h]);
+        }
+        near_level<K, r - 1, LAST>(a, p0, p1);
+    }
+}
+
+// Squared distances of the nearest point of both halves of every bit, for
+// two symbols (p[i][v][b]: symbol i, half v), from a table sorted by label
+// (re, re, im, im).  With one prior for all points the metric falls with the
+// squared distance, and rounding keeps that order, so the maximum metric is
+// the metric of the smallest distance, bit for bit: a point costs its
+// distance (five two-lane operations for two symbols) and two minima a symbol
+// in place of seven operations and 2.6 maxima.  Two halves of a chunk of 32
+// are folded as the second is formed, so 16 distances per symbol are held.
+template <int K>
+__device__ __forceinline__ void nearest_tree(const float4* __restrict__ tab, uint64_t X, uint64_t Y, uint64_t nz,
+                                             float (&p)[2][2][K]) {
+    constexpr int R = K < 5 ? K : 5;   // label bits resolved inside a chunk
+    constexpr int H = R == 5 ? 16 : 1 << R;
+    constexpr int L = 1 << K;
+    const auto distance = [&](int l, float& a, float& b) {
+        const float4 q = tab[l];
+        const uint64_t dr = sub2(X, pk2(q.x, q.y)), di = sub2(Y, pk2(q.z, q.w));
+        upk2(add2(mul2z(dr, dr, nz), mul2z(di, di, nz)), a, b);
+    };
+#pragma unroll 1
+    for (int l0 = 0; l0 < L; l0 += 1 << R) {
+        float a[2][H];
+#pragma unroll
+        for (int j = 0; j < H; ++j) distance(l0 + j, a[0][j], a[1][j]);
+        if constexpr (R == 5) {
+#pragma unroll
+            for (int j = 0; j < H; j += 2) {
+                float c[2][2];
+                distance(l0 + H + j, c[0][0], c[1][0]);
+                distance(l0 + H + j + 1, c[0][1], c[1][1]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    p[i][0][K - 5] = min3(p[i][0][K - 5], a[i][j], a[i][j + 1]);
+                    p[i][1][K - 5] = min3(p[i][1][K - 5], c[i][0], c[i][1]);
+                    a[i][j] = fminf(a[i][j], c[i][0]);
+                    a[i][j + 1] = fminf(a[i][j + 1], c[i][1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            near_level<K, (R == 5 ? 3 : R - 1), (K > 5)>(a[i], p[i][0], p[i][1]);
+            // a[i][0] is the chunk's minimum; its labels share bits 5 and above.
+#pragma unroll
+            for (int q = R; q < K; ++q) {
+                if ((l0 >> q) & 1)
+                    p[i][1][K - 1 - q] = fminf(p[i][1][K - 1 - q], a[i][0]);
+                else
+                    p[i][0][K - 1 - q] = fminf(p[i][0][K - 1 - q], a[i][0]);
+            }
         }
     }
 }
@@ -380,7 +470,10 @@ __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __re
                                                               float* __restrict__ out, bool vec) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int L = 1 << K;
-    __shared__ int s_bad, s_ident;
+    using C = Cross<K>;
+    __shared__ int s_bad, s_ident, s_same, s_cross;
+    __shared__ __align__(16) float2 s_lev[2][(C::N + 1) / 2 * 2];  // the cross's coordinates, each twice
+    __shared__ __align__(8) float s_nz[2];
     const uint32_t stride = gridDim.x * blockDim.x;
     if constexpr (SMEM) {
         float4* tab = reinterpret_cast<float4*>(smem);  // max-log: (re, im, log P, -) by label
@@ -391,7 +484,8 @@ __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __re
         uint32_t* seen = reinterpret_cast<uint32_t*>(smem + table_bytes(K, EXACT) + 4u * L);
         if (threadIdx.x == 0) {
             s_bad = t.M != L ? 1 : 0;
-            s_ident = 1;
+            s_ident = s_same = s_cross = 1;
+            s_nz[0] = s_nz[1] = -0.0f;
             if (EXACT) nz[0] = nz[1] = -0.0f;
         }
         for (int i = threadIdx.x; i < (L + 31) / 32; i += blockDim.x) seen[i] = 0u;
@@ -412,6 +506,7 @@ __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __re
                 }
                 const float2 p = t.pts[m];
                 const float l = t.logp[m];
+                if (!EXACT && l != t.logp[0]) s_same = 0;
                 if (EXACT) {
                     ri[lab] = make_float4(p.x, p.x, p.y, p.y);
                     lp[lab] = make_float2(l, l);
@@ -441,6 +536,90 @@ __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __re
                 return;
             }
         } else {
+            if (s_bad == 0 && s_same) {
+                // One prior for all points: two symbols per step by distance.
+                const float lp0 = t.logp[0];
+                for (int m = threadIdx.x; m < L; m += blockDim.x) {
+                    const float4 q = tab[m];
+                    tab[m] = make_float4(q.x, q.x, q.y, q.y);
+                    if constexpr (C::kIs) {
+                        s_lev[0][C::re(m)] = make_float2(q.x, q.x);
+                        s_lev[1][C::im(m)] = make_float2(q.y, q.y);
+                    }
+                }
+                __syncthreads();
+                if constexpr (C::kIs) {
+                    // Gray cross QAM, whatever its scale: every point at the
+                    // coordinates of its label's place in the cross.
+                    for (int m = threadIdx.x; m < L; m += blockDim.x)
+                        if (tab[m].x != s_lev[0][C::re(m)].x || tab[m].z != s_lev[1][C::im(m)].x) s_cross = 0;
+                    __syncthreads();
+                }
+                const uint64_t NZ = lds_nz(ck::smem_addr(s_nz));
+                // One 16-byte load per pair up to 4 bits per symbol, two of 8
+                // above (measured at 2^22 symbols: 16-PSK 25 against 27 us,
+                // 32- and 128-cross-QAM 48 and 59 against 32 and 49 us).
+                const bool wide = K <= 4 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+                const uint32_t pairs = n / 2 + (n & 1u);
+                // Symbols 2 q and 2 q + 1 (the last one of an odd count twice),
+                // the next pair requested before the arithmetic.
+                const auto load = [&](uint32_t q) {
+                    if (q >= pairs) return make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (wide && 2u * q + 1u < n) return ld_stream(reinterpret_cast<const float4*>(x) + q);
+                    const float2 a = __ldcs(x + 2u * q), b = 2u * q + 1u < n ? __ldcs(x + 2u * q + 1u) : a;
+                    return make_float4(a.x, a.y, b.x, b.y);
+                };
+                float4 next = load(blockIdx.x * blockDim.x + threadIdx.x);
+                for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < pairs; q += stride) {
+                    const uint32_t i0 = 2u * q;
+                    const bool two = i0 + 1u < n;
+                    const float4 v = next;
+                    next = load(q + stride);
+                    float p[2][2][K];
+#pragma unroll
+                    for (int b = 0; b < K; ++b) p[0][0][b] = p[0][1][b] = p[1][0][b] = p[1][1][b] = CUDART_INF_F;
+                    if (C::kIs && s_cross) {
+                        float d[2][2][C::N];  // per symbol and axis
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+#pragma unroll
+                            for (int j = 0; j < C::N; j += 2) {
+                                const uint64_t xc = c ? pk2(v.y, v.w) : pk2(v.x, v.z);
+                                const float4 l = *reinterpret_cast<const float4*>(&s_lev[c][j]);
+                                const uint64_t d0 = sub2(xc, pk2(l.x, l.y)), d1 = sub2(xc, pk2(l.z, l.w));
+                                upk2(mul2(d0, d0), d[0][c][j], d[1][c][j]);
+                                if constexpr (C::kIs) upk2(mul2(d1, d1), d[0][c][j + 1], d[1][c][j + 1]);
+                            }
+                        if constexpr (C::kIs) {
+                            cross_halves<K>(d[0][0], d[0][1], p[0]);
+                            cross_halves<K>(d[1][0], d[1][1], p[1]);
+                        }
+                    } else {
+                        nearest_tree<K>(tab, pk2(v.x, v.z), pk2(v.y, v.w), NZ, p);
+                    }
+                    float sa, sb;
+                    if (two)
+                        noise.pair(i0, sa, sb);
+                    else
+                        sa = sb = noise.at(i0);
+                    const uint64_t ns2 = pk2(-sa, -sb), lp2 = pk2(lp0, lp0);
+                    float o[2 * K];
+#pragma unroll
+                    for (int b = 0; b < K; ++b) {
+                        const uint64_t m0 = add2(mul2z(pk2(p[0][0][b], p[1][0][b]), ns2, NZ), lp2);
+                        const uint64_t m1 = add2(mul2z(pk2(p[0][1][b], p[1][1][b]), ns2, NZ), lp2);
+                        upk2(sub2(m0, m1), o[b], o[K + b]);
+                    }
+                    float* row = out + static_cast<uint64_t>(i0) * K;
+                    if (vec && two)
+                        store_row<2 * K>(row, o, true);
+                    else {
+                        store_row<K>(row, o, false);
+                        if (two) store_row<K>(row + K, o + K, false);
+                    }
+                }
+                return;
+            }
             // Max-log from any staged table (order-free), one symbol per step.
             if (s_bad == 0) {
                 for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
