@@ -139,9 +139,18 @@ struct Resolved {
     int32_t sign_words;  // wide min-sum state: sign words per row (0: packed or sum-product)
     bool edges;  // min-sum with one message per edge in shared memory (CK_LDPC_PLACE_EDGES)
     bool ell;    // decode_ell_kernel
+    // The register form of a code that keeps one message per edge (null:
+    // none): its threads per frame, shared memory and blocks per SM.
+    const void* reg_kernel;
+    int32_t reg_T;
+    uint32_t reg_smem;
+    int reg_per_sm;
+    bool direct;  // a block per frame, all resident: no queue
 };
 
 constexpr int kMaxCluster = 8;  // the portable cluster size
+constexpr uint32_t kRegAppOffset = 128;  // the posterior's place in the register form's shared memory
+constexpr int kRegWaves = 8;             // most waves of frames it takes (ck_ldpc_regs.cuh has the figures)
 
 constexpr size_t kHeaderBytes = 256;
 static_assert(4 * kMaxMixed <= kHeaderBytes, "the mixed launch's queue counters sit in the header");
@@ -223,7 +232,20 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
             }
         }
     }
-    if (r->cluster <= 1 && B > 0 && B < int64_t(sms) * per_sm * G) {
+    // Batches of up to kRegWaves waves: the register form (one frame per
+    // block), where the time of a frame counts for more than the frames an
+    // SM holds.
+    const bool regs = r->reg_kernel && B > 0 && B <= int64_t(sms) * r->reg_per_sm * kRegWaves;
+    r->direct = regs && B <= int64_t(sms) * r->reg_per_sm;
+    if (regs) {
+        r->kernel = r->reg_kernel;
+        r->T = r->reg_T;
+        G = r->G = 1;
+        r->smem = r->reg_smem;
+        r->app_off = kRegAppOffset;
+        per_sm = r->reg_per_sm;
+    }
+    if (!regs && r->cluster <= 1 && B > 0 && B < int64_t(sms) * per_sm * G) {
         // Less than one resident wave: spread the frames over every resident
         // block (fewer frame groups per block, the same kernel) instead of
         // filling the first blocks and leaving SMs idle.  Any shape gives the
@@ -449,6 +471,22 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
     r->cluster_per_sm = 0;
     r->cluster = 1;
     r->ell = ell;
+    r->reg_kernel = nullptr;
+    if (edge_kernel && plan->launch.threads_per_frame == 0 && plan->launch.frames_per_block == 0 &&
+        register_threads(*plan) > 0) {
+        const void* special = nullptr;
+        if (may_compile)
+            CK_TRY(specialised_kernel(plan, kernel_dmax(true, plan->max_deg), kPlaceRegisters, &special));
+        else
+            CK_TRY(specialised_kernel_ready(plan, kPlaceRegisters, &special));
+        if (special) {
+            r->reg_T = register_threads(*plan);
+            r->reg_smem = kRegAppOffset + static_cast<uint32_t>(plan->N + r->reg_T) * 4;
+            CK_TRY(ck::allow_max_smem(special, plan->device, optin));
+            CK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r->reg_per_sm, special, r->reg_T, r->reg_smem));
+            if (r->reg_per_sm > 0) r->reg_kernel = special;
+        }
+    }
     if (!plan->qc && !ell && !app_smem && !r_smem) {
         KernelFn ck = sp ? sum_product_cluster_kernel(plan->max_deg) : min_sum_cluster_kernel(plan->max_deg);
         int cps = 0;
@@ -591,6 +629,7 @@ Params make_params(const ck_ldpc_plan* plan, const Resolved& r, const float* llr
     p.ell_info = reinterpret_cast<const uint32_t*>(plan->d_ell_info);
     p.ell_rows = static_cast<uint32_t>(plan->ell_rows);
     p.ell_ns = plan->ell_ns;
+    p.direct = r.direct ? 1 : 0;
     if (r.ell) p.m = plan->ell_rows;
     return p;
 }
@@ -635,7 +674,7 @@ extern "C" int ck_ldpc_decode(const ck_ldpc_plan* plan, const float* llr_in, flo
             return ck::fail(CK_ERR_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
     }
     unsigned char* wsb = static_cast<unsigned char*>(ws);
-    int status = ck::cuda_check(cudaMemsetAsync(wsb, 0, kHeaderBytes, s), "cudaMemsetAsync");
+    int status = r.direct ? CK_OK : ck::cuda_check(cudaMemsetAsync(wsb, 0, kHeaderBytes, s), "cudaMemsetAsync");
     const Params p = make_params(plan, r, llr_in, llr_out, B, n_in, scale, offset, max_iterations,
                                  early_stop, iters, valid, bits, k_bits, wsb);
     if (status == CK_OK) status = launch_decode(r, p, s);

@@ -70,7 +70,7 @@ struct ck_ldpc_plan {
         ck_ldpc_launch launch{0, 0, 0};
         int32_t jit_mode = 0;
         int per_sm = 0, sms = 0;
-        alignas(16) unsigned char resolved[224];
+        alignas(16) unsigned char resolved[256];
     };
     mutable ShapeCache shape_cache[2];
     mutable std::mutex shape_mu;
@@ -80,7 +80,7 @@ struct ck_ldpc_plan {
         bool tried = false;
         int dmax = 0;
         cudaLibrary_t lib = nullptr;
-        const void* kernel[3] = {nullptr, nullptr, nullptr};  // by placement: device, records, edges
+        const void* kernel[4] = {nullptr, nullptr, nullptr, nullptr};  // by placement: device, records, edges, registers
         std::string why;  // why there are none
     };
     uint64_t id = 0;  // unique in the process, never reused
@@ -103,6 +103,12 @@ namespace ldpc {
 constexpr int kPlaceDevice = 0;  // packed records in device memory
 constexpr int kPlaceRecords = 1;  // packed records in shared memory
 constexpr int kPlaceEdges = 2;  // one message per edge in shared memory
+constexpr int kPlaceRegisters = 3;  // one message per edge in registers (decode_regs_body)
+// Threads per frame of a circulant plan's register form (two lanes per row,
+// whole warps of 16 rows), or 0 where it has none: more than kRegSlots edges
+// per lane, or a longest row above kPackedDegree.
+constexpr int kRegSlots = 72;
+int32_t register_threads(const ck_ldpc_plan& plan);
 // The plan's code-specialised min-sum kernel for a row-degree bound and a
 // message-state placement (compiled on first use), or nullptr in *out when
 // the plan has none (specialisation off, NVRTC missing or the compilation

@@ -306,13 +306,104 @@ std::string program_struct(const ck_ldpc_plan& plan, const char* name, int H = 1
     return s;
 }
 
+// Edge slots per lane of the register form: half of each base row's edges.
+int register_slots(const ck_ldpc_plan& plan) {
+    int slots = 0;
+    for (int32_t b = 0; b < plan.mb; ++b) slots += (plan.h_eptr[b + 1] - plan.h_eptr[b] + 1) / 2;
+    return slots;
+}
+
+// The program of the register form (decode_regs_body): base row b's edges
+// 0 .. D0 - 1 on the lower lanes, the rest on the upper ones, in the slots
+// from slot[b] on.
+std::string registers_struct(const ck_ldpc_plan& plan, const char* name) {
+    const int32_t Z = plan.Z;
+    std::vector<int32_t> slot(plan.mb + 1, 0), half(plan.mb);
+    for (int32_t b = 0; b < plan.mb; ++b) {
+        half[b] = (plan.h_eptr[b + 1] - plan.h_eptr[b] + 1) / 2;
+        slot[b + 1] = slot[b] + half[b];
+    }
+    std::string s = std::string("struct ") + name + " {\n";
+    add(s, "    static constexpr int kSlots = %lld;\n", slot[plan.mb]);
+    s += "    __device__ __forceinline__ static void columns(uint32_t* a, const uint32_t a_addr, const uint32_t r, const int h,\n";
+    s += "                                                   const uint32_t own) {\n";
+    s += "        const auto at = [&](uint32_t first, uint32_t end) {\n";  // (j Z + shift, (j + 1) Z), as the plan's tables
+    add(s, "            const uint32_t c = r + first;\n            return a_addr + 4u * (c >= end ? c - %lldu : c);\n        };\n", Z);
+    add(s, "        const bool row = r < %lldu;\n", Z);
+    for (int32_t b = 0; b < plan.mb; ++b) {
+        const int32_t e0 = plan.h_eptr[b], D = plan.h_eptr[b + 1] - e0;
+        for (int32_t i = 0; i < half[b]; ++i) {
+            const int32_t lo = e0 + i, hi = e0 + half[b] + i;
+            add(s, "        a[%lld] = !row ? own : h == 0 ? at(%lldu, %lldu)", slot[b] + i, plan.h_blk[2 * lo],
+                plan.h_blk[2 * lo + 1]);
+            if (half[b] + i < D)
+                add(s, " : at(%lldu, %lldu);\n", plan.h_blk[2 * hi], plan.h_blk[2 * hi + 1]);
+            else
+                s += " : own;\n";
+        }
+    }
+    s += "    }\n";
+    s += "    __device__ __forceinline__ static void clear(float* m) {\n";
+    for (int32_t k = 0; k < slot[plan.mb]; ++k) add(s, "        m[%lld] = 0.0f;\n", k);
+    s += "    }\n";
+    s += "    __device__ __forceinline__ static void iteration(float* m, const uint32_t* a, const float scale, const float offset,\n";
+    s += "                                                     const int T) {\n";
+    for (int32_t l = 0; l < plan.L; ++l) {
+        add(s, "        {  // layer %lld\n", l);
+        for (int32_t b = plan.h_layer[l]; b < plan.h_layer[l + 1]; ++b) {
+            add(s, "            float q%lld[%lld];\n", b, half[b]);
+            for (int32_t i = 0; i < half[b]; ++i)
+                add(s, "            q%lld[%lld] = ld_shared_f32(a[%lld]);\n", b, i, slot[b] + i);
+        }
+        for (int32_t b = plan.h_layer[l]; b < plan.h_layer[l + 1]; ++b) {
+            for (int32_t i = 0; i < half[b]; ++i) {
+                add(s, "            q%lld[%lld] = __fsub_rn(q%lld", b, i, b);
+                add(s, "[%lld], m[%lld]);\n", i, slot[b] + i);
+            }
+            add(s, "            const RegRow r%lld = reg_row_minima<%lld>(q%lld);\n", b, half[b], b);
+        }
+        for (int32_t b = plan.h_layer[l]; b < plan.h_layer[l + 1]; ++b) {
+            add(s, "            const RegOut o%lld = reg_row_out(r%lld, scale, offset);\n", b, b);
+            for (int32_t i = 0; i < half[b]; ++i) {
+                add(s, "            reg_edge(o%lld, q%lld[%lld], ", b, b, i);
+                add(s, "a[%lld], m[%lld]);\n", slot[b] + i, slot[b] + i);
+            }
+        }
+        s += "            ck::group_sync(1, T);\n        }\n";
+    }
+    s += "    }\n";
+    // The first base row by itself (an unconverged frame usually fails
+    // there), then the others.
+    s += "    __device__ __forceinline__ static bool syndrome(const uint32_t* a, const int T) {\n";
+    s += "        uint32_t bad = 0u;\n";
+    for (int32_t b = 0; b < plan.mb; ++b) {
+        s += "        {\n            uint32_t x = 0u;\n";
+        for (int32_t i = 0; i < half[b]; ++i)
+            add(s, "            x ^= __float_as_uint(ld_shared_f32(a[%lld]));\n", slot[b] + i);
+        s += "            x ^= __shfl_xor_sync(0xffffffffu, x, 16);\n            bad |= x >> 31;\n        }\n";
+        if (b == 0 || b + 1 == plan.mb) s += "        if (ck::group_any(static_cast<int>(bad), 1, T)) return false;\n";
+    }
+    s += "        return true;\n    }\n};\n";
+    return s;
+}
+
 // The plain decoder of one code: one kernel per message-state placement
 // (r0 records in device memory, r1 records in shared memory, r2 one
-// message per edge in shared memory).
+// message per edge in shared memory, r3 in registers where the code has
+// that form).
 std::string program_source(const ck_ldpc_plan& plan, int dmax) {
-    std::string s = "#include \"ck_ldpc_minsum.cuh\"\nusing namespace ck::ldpc;\nnamespace {\n";
+    const int32_t reg_threads = register_threads(plan);
+    std::string s = "#include \"ck_ldpc_regs.cuh\"\nusing namespace ck::ldpc;\nnamespace {\n";
     s += program_struct(plan, "CodeProgram");
+    if (reg_threads) s += registers_struct(plan, "RegisterProgram");
     s += "}  // namespace\n";
+    if (reg_threads) {
+        // Two registers per slot and about 40 more; the blocks that leaves.
+        const int regs = (2 * register_slots(plan) + 40 + 7) / 8 * 8;
+        add(s, "extern \"C\" __global__ void __launch_bounds__(%lld, %lld) ck_ldpc_code_r3(const __grid_constant__ Params p) {\n",
+            reg_threads, std::max(1, std::min(65536 / (regs * reg_threads), 16)));
+        s += "    decode_regs_body<RegisterProgram>(p);\n}\n";
+    }
     for (int r = 0; r < 3; ++r) {
         // A minimum of one block per SM, stated: without it ptxas held some of
         // these kernels to 40 registers and spilled.
@@ -449,6 +540,12 @@ std::map<std::vector<uint64_t>, MixedJit> g_mixed;
 
 }  // namespace
 
+int32_t register_threads(const ck_ldpc_plan& plan) {
+    if (!plan.qc || plan.max_deg > kPackedDegree || register_slots(plan) > kRegSlots) return 0;
+    const int32_t T = (plan.Z + 15) / 16 * 32;
+    return T <= 512 ? T : 0;
+}
+
 std::string specialised_source(const ck_ldpc_plan& plan, int dmax) { return program_source(plan, dmax); }
 
 std::string mixed_source(const ck_ldpc_plan* const* plans, const int* parts, const int* edges, int n, int dmax) {
@@ -464,8 +561,9 @@ int specialised_kernel(const ck_ldpc_plan* plan, int dmax, int place, const void
     if (!j.tried) {  // a plan's degree bound never changes, so one compilation serves it
         j.tried = true;
         j.dmax = dmax;
-        static const char* const names[] = {"ck_ldpc_code_r0", "ck_ldpc_code_r1", "ck_ldpc_code_r2"};
-        if (!compile_load(program_source(*plan, dmax), plan->device, names, 3, &j.lib, j.kernel, &j.why))
+        static const char* const names[] = {"ck_ldpc_code_r0", "ck_ldpc_code_r1", "ck_ldpc_code_r2", "ck_ldpc_code_r3"};
+        if (!compile_load(program_source(*plan, dmax), plan->device, names, register_threads(*plan) ? 4 : 3, &j.lib,
+                          j.kernel, &j.why))
             j.lib = nullptr;
     }
     if (!j.lib) {
@@ -555,7 +653,8 @@ void forget_plan_kernels(const ck_ldpc_plan* plan) {
         it = g_mixed.erase(it);
     }
     if (plan->jit.lib) {
-        for (const void* k : plan->jit.kernel) ck::forget_kernel(k);
+        for (const void* k : plan->jit.kernel)
+            if (k) ck::forget_kernel(k);
         (void)cudaLibraryUnload(plan->jit.lib);
     }
 }

@@ -75,6 +75,9 @@ struct Params {
     const uint32_t* ell_info;
     uint32_t ell_rows;
     int32_t ell_ns;
+    // The register form with a block per frame: block f decodes frame f, no
+    // queue (the workspace header is not zeroed before the launch).
+    int32_t direct;
 };
 
 __device__ __forceinline__ float flip_sign(float v, uint32_t bit) {

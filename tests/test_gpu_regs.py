@@ -1,0 +1,58 @@
+"""Min-sum batches of the register form (two lanes per row, messages and
+columns in registers) against the CPU oracle, bit for bit: liftings around
+its 16-row warps, rows of odd and even degree, codes at and above its edge
+slots, batches of one frame, of a block per frame and of several waves."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+from commkit_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+# mb, nb, Z, information column weights, punctured, frames.
+CASES = [
+    (4, 8, 2, 2, 0, 1),
+    (3, 7, 15, 2, 0, 5),
+    (5, 11, 16, 3, 3, 33),
+    (6, 12, 17, 3, 0, 153),
+    (12, 24, 54, 4, 0, 700),
+    (12, 24, 54, 4, 1, 5200),
+    (6, 24, 96, 3, 0, 1300),
+    (4, 30, 31, 4, 0, 64),  # rows of 27 edges
+    (16, 48, 8, 3, 0, 300),  # 72 slots: about the limit
+    (20, 60, 8, 3, 0, 300),  # beyond it
+    (4, 9, 256, 2, 0, 40),
+    (4, 9, 257, 2, 0, 40),  # beyond its threads
+]
+
+
+@pytest.mark.parametrize("mb,nb,z,weight,punctured,frames", CASES)
+def test_circulant_codes_equal_oracle(mb, nb, z, weight, punctured, frames):
+    import torch
+
+    import commkit_gb300 as ck
+    from commkit_gb300 import _device, _lib
+
+    base = W.dual_diagonal_base(mb, nb, z, (weight,) * (nb - mb), seed=z)
+    code = ck.LDPCCode.quasi_cyclic(base, lifting=z, punctured=punctured)
+    rng = np.random.default_rng(3)
+    llrs = (2.0 + 2.2 * rng.standard_normal((frames, code.n))).astype(np.float32)
+    llrs[0, :6] = [0.0, -0.0, np.inf, -np.inf, 1e30, np.nan]
+    x = torch.from_numpy(llrs).cuda()
+    row_ptr, cols, _ = code._schedule
+    for method in (ck.MinSum(max_iterations=9), ck.MinSum(scale=0.75, offset=0.05, max_iterations=3, early_stop=False)):
+        want = oracle.decode(llrs, (row_ptr, cols, code.num_variables), k=code.k, scale=method.scale,
+                             offset=method.offset, max_iterations=method.max_iterations,
+                             early_stop=method.early_stop)  # fmt: skip
+        # The caller's workspace as it comes: its header is not zeroed.
+        ws = torch.full((code._plan(0).workspace_size(frames),), 255, dtype=torch.uint8, device="cuda")
+        for r in (ck.decode(x, code=code, method=method), ck.decode(x, code=code, method=method, workspace=ws)):
+            got = (r.bits, r.llrs, r.valid, r.iterations)
+            for g, w, what in zip(got, want, ("bits", "llrs", "valid", "iterations"), strict=True):
+                np.testing.assert_array_equal(g.cpu().numpy().reshape(w.shape), w, err_msg=what)
+        wd = _device.wrap(ws)
+        assert _lib.lib().ck_ldpc_workspace_status(wd.ptr, _device.stream_of(wd)) == _lib.CK_OK
