@@ -139,8 +139,7 @@ struct Resolved {
     int32_t sign_words;  // wide min-sum state: sign words per row (0: packed or sum-product)
     bool edges;  // min-sum with one message per edge in shared memory (CK_LDPC_PLACE_EDGES)
     bool ell;    // decode_ell_kernel
-    // The register form of a code that keeps one message per edge (null:
-    // none): its threads per frame, shared memory and blocks per SM.
+    // The register form of a code that has one (null: none): its threads per frame, shared memory and blocks per SM.
     const void* reg_kernel;
     int32_t reg_T;
     uint32_t reg_smem;
@@ -150,7 +149,7 @@ struct Resolved {
 
 constexpr int kMaxCluster = 8;  // the portable cluster size
 constexpr uint32_t kRegAppOffset = 128;  // the posterior's place in the register form's shared memory
-constexpr int kRegWaves = 8;             // most waves of frames it takes (ck_ldpc_regs.cuh has the figures)
+constexpr int kRegWaves = 8;             // most min-sum waves it takes (ck_ldpc_regs.cuh has the figures)
 
 constexpr size_t kHeaderBytes = 256;
 static_assert(4 * kMaxMixed <= kHeaderBytes, "the mixed launch's queue counters sit in the header");
@@ -232,10 +231,11 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
             }
         }
     }
-    // Batches of up to kRegWaves waves: the register form (one frame per
-    // block), where the time of a frame counts for more than the frames an
-    // SM holds.
-    const bool regs = r->reg_kernel && B > 0 && B <= int64_t(sms) * r->reg_per_sm * kRegWaves;
+    // The register form (one frame per block): sum-product batches of every
+    // size, min-sum batches of up to kRegWaves waves, where the time of a
+    // frame counts for more than the frames an SM holds.
+    const bool regs = r->reg_kernel && B > 0 &&
+                      (rule == CK_LDPC_SUM_PRODUCT || B <= int64_t(sms) * r->reg_per_sm * kRegWaves);
     r->direct = regs && B <= int64_t(sms) * r->reg_per_sm;
     if (regs) {
         r->kernel = r->reg_kernel;
@@ -472,10 +472,12 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
     r->cluster = 1;
     r->ell = ell;
     r->reg_kernel = nullptr;
-    if (edge_kernel && plan->launch.threads_per_frame == 0 && plan->launch.frames_per_block == 0 &&
+    if ((sp || (edge_kernel && plan->launch.frames_per_block == 0)) && plan->launch.threads_per_frame == 0 &&
         register_threads(*plan) > 0) {
         const void* special = nullptr;
-        if (may_compile)
+        if (sp)
+            special = sum_product_register_kernel(plan, may_compile);
+        else if (may_compile)
             CK_TRY(specialised_kernel(plan, kernel_dmax(true, plan->max_deg), kPlaceRegisters, &special));
         else
             CK_TRY(specialised_kernel_ready(plan, kPlaceRegisters, &special));

@@ -86,6 +86,7 @@ struct ck_ldpc_plan {
     uint64_t id = 0;  // unique in the process, never reused
     int32_t jit_mode = CK_LDPC_SPECIALISE_AUTO;
     mutable Jit jit;
+    mutable Jit jit_sp;  // the sum-product register form, compiled on its first use
     mutable std::mutex jit_mu;
 };
 
@@ -114,6 +115,10 @@ int32_t register_threads(const ck_ldpc_plan& plan);
 // the plan has none (specialisation off, NVRTC missing or the compilation
 // failed); an error only when the plan requires specialisation.
 int specialised_kernel(const ck_ldpc_plan* plan, int dmax, int place, const void** out);
+// The plan's sum-product kernel in the register form, or nullptr where it has
+// none (the table-driven kernel then serves); may_compile false: only one
+// that is compiled already.
+const void* sum_product_register_kernel(const ck_ldpc_plan* plan, bool may_compile);
 // The same kernel only if an earlier call already compiled it (nullptr in
 // *out otherwise): never compiles or loads code, for the allocation-free
 // entry point.  An error only when the plan requires specialisation and has

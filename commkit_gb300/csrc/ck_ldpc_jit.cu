@@ -316,7 +316,7 @@ int register_slots(const ck_ldpc_plan& plan) {
 // The program of the register form (decode_regs_body): base row b's edges
 // 0 .. D0 - 1 on the lower lanes, the rest on the upper ones, in the slots
 // from slot[b] on.
-std::string registers_struct(const ck_ldpc_plan& plan, const char* name) {
+std::string registers_struct(const ck_ldpc_plan& plan, const char* name, bool sum_product) {
     const int32_t Z = plan.Z;
     std::vector<int32_t> slot(plan.mb + 1, 0), half(plan.mb);
     for (int32_t b = 0; b < plan.mb; ++b) {
@@ -356,16 +356,30 @@ std::string registers_struct(const ck_ldpc_plan& plan, const char* name) {
                 add(s, "            q%lld[%lld] = ld_shared_f32(a[%lld]);\n", b, i, slot[b] + i);
         }
         for (int32_t b = plan.h_layer[l]; b < plan.h_layer[l + 1]; ++b) {
+            if (sum_product) add(s, "            float f%lld[%lld];\n", b, half[b]);
             for (int32_t i = 0; i < half[b]; ++i) {
                 add(s, "            q%lld[%lld] = __fsub_rn(q%lld", b, i, b);
                 add(s, "[%lld], m[%lld]);\n", i, slot[b] + i);
+                if (sum_product) {
+                    add(s, "            f%lld[%lld] = reg_phi(fabsf(q%lld", b, i, b);
+                    add(s, "[%lld]));\n", i);
+                }
             }
-            add(s, "            const RegRow r%lld = reg_row_minima<%lld>(q%lld);\n", b, half[b], b);
+            if (sum_product)
+                add(s, "            const RegSum r%lld = reg_row_total<%lld>(q%lld, ", b, half[b], b);
+            else
+                add(s, "            const RegRow r%lld = reg_row_minima<%lld>(q%lld);\n", b, half[b], b);
+            if (sum_product) add(s, "f%lld, (threadIdx.x & 16) != 0);\n", b);
         }
         for (int32_t b = plan.h_layer[l]; b < plan.h_layer[l + 1]; ++b) {
-            add(s, "            const RegOut o%lld = reg_row_out(r%lld, scale, offset);\n", b, b);
+            if (!sum_product) add(s, "            const RegOut o%lld = reg_row_out(r%lld, scale, offset);\n", b, b);
             for (int32_t i = 0; i < half[b]; ++i) {
-                add(s, "            reg_edge(o%lld, q%lld[%lld], ", b, b, i);
+                if (sum_product) {
+                    add(s, "            reg_sp_edge(r%lld, q%lld[%lld], ", b, b, i);
+                    add(s, "f%lld[%lld], ", b, i);
+                } else {
+                    add(s, "            reg_edge(o%lld, q%lld[%lld], ", b, b, i);
+                }
                 add(s, "a[%lld], m[%lld]);\n", slot[b] + i, slot[b] + i);
             }
         }
@@ -387,6 +401,21 @@ std::string registers_struct(const ck_ldpc_plan& plan, const char* name) {
     return s;
 }
 
+// The register form's kernel: two registers per slot and about 40 more, and
+// the blocks per SM that leaves.
+std::string registers_kernel(const ck_ldpc_plan& plan, const char* name) {
+    const int T = register_threads(plan), regs = (2 * register_slots(plan) + 40 + 7) / 8 * 8;
+    std::string s;
+    add(s, "extern \"C\" __global__ void __launch_bounds__(%lld, %lld) ", T, std::max(1, std::min(65536 / (regs * T), 16)));
+    return s + name + "(const __grid_constant__ Params p) {\n    decode_regs_body<RegisterProgram>(p);\n}\n";
+}
+
+// The sum-product decoder of one code in the register form.
+std::string sum_product_source(const ck_ldpc_plan& plan) {
+    return "#include \"ck_ldpc_regs.cuh\"\nusing namespace ck::ldpc;\nnamespace {\n" +
+           registers_struct(plan, "RegisterProgram", true) + "}  // namespace\n" + registers_kernel(plan, "ck_ldpc_code_sp");
+}
+
 // The plain decoder of one code: one kernel per message-state placement
 // (r0 records in device memory, r1 records in shared memory, r2 one
 // message per edge in shared memory, r3 in registers where the code has
@@ -395,15 +424,9 @@ std::string program_source(const ck_ldpc_plan& plan, int dmax) {
     const int32_t reg_threads = register_threads(plan);
     std::string s = "#include \"ck_ldpc_regs.cuh\"\nusing namespace ck::ldpc;\nnamespace {\n";
     s += program_struct(plan, "CodeProgram");
-    if (reg_threads) s += registers_struct(plan, "RegisterProgram");
+    if (reg_threads) s += registers_struct(plan, "RegisterProgram", false);
     s += "}  // namespace\n";
-    if (reg_threads) {
-        // Two registers per slot and about 40 more; the blocks that leaves.
-        const int regs = (2 * register_slots(plan) + 40 + 7) / 8 * 8;
-        add(s, "extern \"C\" __global__ void __launch_bounds__(%lld, %lld) ck_ldpc_code_r3(const __grid_constant__ Params p) {\n",
-            reg_threads, std::max(1, std::min(65536 / (regs * reg_threads), 16)));
-        s += "    decode_regs_body<RegisterProgram>(p);\n}\n";
-    }
+    if (reg_threads) s += registers_kernel(plan, "ck_ldpc_code_r3");
     for (int r = 0; r < 3; ++r) {
         // A minimum of one block per SM, stated: without it ptxas held some of
         // these kernels to 40 registers and spilled.
@@ -542,6 +565,8 @@ std::map<std::vector<uint64_t>, MixedJit> g_mixed;
 
 int32_t register_threads(const ck_ldpc_plan& plan) {
     if (!plan.qc || plan.max_deg > kPackedDegree || register_slots(plan) > kRegSlots) return 0;
+    for (int32_t b = 0; b < plan.mb; ++b)
+        if (plan.h_eptr[b + 1] == plan.h_eptr[b]) return 0;  // a lane's part of a row is an array
     const int32_t T = (plan.Z + 15) / 16 * 32;
     return T <= 512 ? T : 0;
 }
@@ -573,6 +598,18 @@ int specialised_kernel(const ck_ldpc_plan* plan, int dmax, int place, const void
     }
     *out = j.kernel[place];
     return CK_OK;
+}
+
+const void* sum_product_register_kernel(const ck_ldpc_plan* plan, bool may_compile) {
+    if (register_threads(*plan) == 0 || effective_mode(plan->jit_mode) == CK_LDPC_SPECIALISE_OFF) return nullptr;
+    std::lock_guard<std::mutex> lock(plan->jit_mu);
+    ck_ldpc_plan::Jit& j = plan->jit_sp;
+    if (!j.tried && may_compile) {
+        j.tried = true;
+        static const char* const names[] = {"ck_ldpc_code_sp"};
+        if (!compile_load(sum_product_source(*plan), plan->device, names, 1, &j.lib, j.kernel, &j.why)) j.lib = nullptr;
+    }
+    return j.lib ? j.kernel[0] : nullptr;
 }
 
 int specialised_kernel_ready(const ck_ldpc_plan* plan, int place, const void** out) {
@@ -656,6 +693,10 @@ void forget_plan_kernels(const ck_ldpc_plan* plan) {
         for (const void* k : plan->jit.kernel)
             if (k) ck::forget_kernel(k);
         (void)cudaLibraryUnload(plan->jit.lib);
+    }
+    if (plan->jit_sp.lib) {
+        ck::forget_kernel(plan->jit_sp.kernel[0]);
+        (void)cudaLibraryUnload(plan->jit_sp.lib);
     }
 }
 

@@ -1,0 +1,66 @@
+"""Sum-product decoding in the register form (two lanes per row, messages in
+registers) against the table-driven kernel, bit for bit: liftings around its
+16-row warps, rows of two, odd and many edges, one frame, a
+block per frame and several waves."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from commkit_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+# mb, nb, Z, information column weights, frames.
+CASES = [
+    (4, 8, 2, 2, 1),
+    (3, 7, 15, 2, 5),
+    (5, 11, 16, 3, 33),
+    (6, 12, 17, 3, 153),
+    (12, 24, 54, 4, 5200),
+    (6, 24, 96, 3, 1300),
+    (4, 30, 31, 4, 64),  # rows of 27 edges
+    (16, 48, 8, 3, 300),  # about the most edge slots
+    (4, 9, 256, 2, 40),  # the most threads
+    (4, 9, 257, 2, 40),  # beyond them
+]
+
+
+def _run(base, z, frames):
+    import torch
+
+    import commkit_gb300 as ck
+    from commkit_gb300 import _lib
+
+    rng = np.random.default_rng(3)
+    got = []
+    for mode in (_lib.CK_LDPC_SPECIALISE_OFF, _lib.CK_LDPC_SPECIALISE_AUTO):
+        code = ck.LDPCCode.quasi_cyclic(base, lifting=z)
+        code._plan(0).set_specialise(mode)
+        if not got:
+            llrs = (2.0 + 2.2 * rng.standard_normal((frames, code.n))).astype(np.float32)
+            llrs[0, :6] = [0.0, -0.0, np.inf, -np.inf, 1e30, np.nan]
+            x = torch.from_numpy(llrs).cuda()
+        out = []
+        for method in (ck.SumProduct(max_iterations=7), ck.SumProduct(max_iterations=3, early_stop=False)):
+            ws = torch.full((code._plan(0).workspace_size(frames, _lib.CK_LDPC_SUM_PRODUCT),), 255, dtype=torch.uint8,
+                            device="cuda")  # fmt: skip
+            for r in (ck.decode(x, code=code, method=method), ck.decode(x, code=code, method=method, workspace=ws)):
+                out += [r.bits, r.llrs, r.valid, r.iterations]
+        got.append([o.cpu().numpy() for o in out])
+    for want, have in zip(*got, strict=True):
+        if want.dtype == np.float32:
+            want, have = want.view(np.uint32), have.view(np.uint32)
+        np.testing.assert_array_equal(have, want)
+
+
+@pytest.mark.parametrize("mb,nb,z,weight,frames", CASES)
+def test_equals_table_kernel(mb, nb, z, weight, frames):
+    _run(W.dual_diagonal_base(mb, nb, z, (weight,) * (nb - mb), seed=z), z, frames)
+
+
+def test_row_of_two_edges():
+    base = W.dual_diagonal_base(6, 12, 17, (3,) * 6, seed=1)
+    base[4, :6] = -1
+    _run(base, 17, 40)
