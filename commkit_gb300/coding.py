@@ -789,20 +789,25 @@ def encode_blocks(code: LDPCCode, info: Any, words: Any = None, scratch: Any = N
         scratch = _device.empty(xd, (e.scratch_bytes(R, m, k),), np.int8)
     sd = _device.wrap(scratch, "scratch")
     with _device.on_device(xd):
-        if e.generator is not None:
-            info_cols, piv, gen = _encoder_tables(code, xd)
-            st = _lib.lib().ck_ldpc_encode_generator(
-                xd.ptr, R, k, e.generator[1].size, n, _device.wrap(info_cols).ptr, _device.wrap(piv).ptr,
-                _device.wrap(gen).ptr, sd.ptr, sd.size, wd.ptr, _device.stream_of(xd),
-            )  # fmt: skip
-        else:
-            rp, ci, inv = _encoder_tables(code, xd)
-            st = _lib.lib().ck_ldpc_encode(
-                xd.ptr, R, k, m, n, _device.wrap(rp).ptr, _device.wrap(ci).ptr, e.stride,
-                None if inv is None else _device.wrap(inv).ptr, sd.ptr, sd.size, wd.ptr, _device.stream_of(xd),
-            )  # fmt: skip
-        _lib.check(st, "encode()")
+        _encode_rows(code, xd, xd.ptr, R, wd.ptr, sd.ptr, sd.size, _device.stream_of(xd))
     return words
+
+
+def _encode_rows(code: LDPCCode, like: _device.DeviceArray, info: int, R: int, words: int, scratch: int,
+                 scratch_bytes: int, stream: int) -> None:  # fmt: skip
+    """The encoder's launch for ``R`` rows at the device addresses ``info``,
+    ``words`` and ``scratch``, on ``like``'s device (the current one)."""
+    ptr = (lambda a: a.data_ptr()) if like.kind == "torch" else (lambda a: _device.wrap(a).ptr)
+    e = code._encoder
+    if e.generator is not None:
+        info_cols, piv, gen = _encoder_tables(code, like)
+        st = _lib.lib().ck_ldpc_encode_generator(info, R, code.k, e.generator[1].size, code.n, ptr(info_cols), ptr(piv),
+                                                 ptr(gen), scratch, scratch_bytes, words, stream)  # fmt: skip
+    else:
+        rp, ci, inv = _encoder_tables(code, like)
+        st = _lib.lib().ck_ldpc_encode(info, R, code.k, code.num_checks, code.n, ptr(rp), ptr(ci), e.stride,
+                                       None if inv is None else ptr(inv), scratch, scratch_bytes, words, stream)  # fmt: skip
+    _lib.check(st, "encode()")
 
 
 def _encode_checked(bits: Any, x: _device.DeviceArray, code: LDPCCode) -> Any:
