@@ -266,6 +266,20 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
             r->smem = r->tables_bytes + static_cast<uint32_t>(g2) * r->group_bytes;
         }
     }
+    if (rule == CK_LDPC_SUM_PRODUCT && !plan->qc && r->app_smem && r->cluster <= 1 && B > 0 &&
+        plan->launch.threads_per_frame == 0 && (B <= sms || per_sm * G == 1)) {
+        // A frame per SM at most, of a code whose posterior is in shared
+        // memory: all the threads the kernel is built for, up to a layer's
+        // rows, since two blocks of 512 would not share the SM.  The phi
+        // calls bound it (DVB-S2 short, 30 iterations
+        // at 2.2 dB: 1 / 32 / 128 frames 520 / 687 / 777 us with 512
+        // threads, 399 / 526 / 588 with 1024; 256 frames, two to an SM, keep 512).
+        const int32_t rows = (plan->max_layer_rows + 31) / 32 * 32;
+        r->T = std::max(r->T, std::min(max_block_threads(false, kernel_dmax(false, plan->max_deg)), rows));
+        G = r->G = 1;
+        r->smem = r->tables_bytes + r->group_bytes;
+        per_sm = 1;
+    }
     const int64_t need = (B + G - 1) / G;
     r->plain_grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * per_sm)));
     if (r->cluster > 1) {
