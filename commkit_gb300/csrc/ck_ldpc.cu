@@ -750,7 +750,10 @@ int ck::ldpc_decode_in_scratch(const ck_ldpc_plan* plan, const float* llr_in, fl
                             "scratch holds %zu",
                             r.G, kHeaderBytes + 256 + per_slot * r.G, scratch_bytes);
         const int grid_cap = static_cast<int>(max_slots / r.G);
-        if (r.grid > grid_cap) r.grid = grid_cap;
+        if (r.grid > grid_cap) {
+            r.grid = grid_cap;
+            r.direct = false;  // fewer blocks than frames: the queue hands them out
+        }
     }
     const size_t slots = static_cast<size_t>(r.grid) * r.G;
     r.r_ws_off = kHeaderBytes;
