@@ -465,8 +465,8 @@ class _Plan:
         return cfg.threads_per_frame, cfg.frames_per_block, cfg.placement
 
     def set_specialise(self, mode: int) -> None:
-        """``_lib.CK_LDPC_SPECIALISE_{AUTO,OFF,ON}``: whether min-sum decodes
-        of this circulant code run its code-specialised kernel."""
+        """``_lib.CK_LDPC_SPECIALISE_{AUTO,OFF,ON}``: whether decodes of
+        this circulant code run its code-specialised kernels."""
         _lib.check(_lib.lib().ck_ldpc_plan_set_specialise(self.handle, int(mode)), "set_specialise")
 
     def specialisation(self) -> tuple[int, int, str]:

@@ -1,4 +1,4 @@
-// Code-specialised min-sum decoders for circulant codes, generated from a
+// Code-specialised decoders for circulant codes, generated from a
 // plan and compiled at run time with NVRTC.
 //
 // The table-driven kernel reads, for every check row, its base row's
@@ -15,7 +15,8 @@
 //
 // Applies to min-sum decodes of circulant codes launched with one frame
 // group thread per row slot (threads per frame == Z rounded up to whole
-// warps).  NVRTC is loaded with dlopen; where it is missing, or a
+// warps), and, in the register form (ck_ldpc_regs.cuh), to short min-sum
+// batches and all sum-product decodes of small codes.  NVRTC is loaded with dlopen; where it is missing, or a
 // compilation fails, decodes keep the table-driven kernel unless the plan
 // requires specialisation.
 #include <dlfcn.h>

@@ -2,7 +2,8 @@
 // reference's `ldpc_layered<true>` (commkit/_cuda/src/ldpc.cu:74-91; CPU twin
 // commkit/coding/_numba_loops.py:71-94) run by the persistent frame loop the
 // min-sum rule uses (ck_ldpc_kernel.cuh): same layers, same order, same
-// early stop.
+// early stop.  Small circulant codes run a generated program instead
+// (ck_ldpc_regs.cuh); this is the kernel of the others.
 //
 // The check-to-variable message of edge e is
 //     sign_e * phi(sum_e' phi(|Q_e'|) - phi(|Q_e|)),   phi(x) = -log tanh(x / 2)

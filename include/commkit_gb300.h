@@ -355,12 +355,14 @@ int ck_ldpc_plan_get_launch(const ck_ldpc_plan* plan, ck_ldpc_launch* launch);
 int ck_ldpc_plan_resolved_launch(const ck_ldpc_plan* plan, int32_t rule, ck_ldpc_launch* launch);
 
 /*
- * Code-specialised min-sum decoding of a circulant code (no reference
+ * Code-specialised decoding of a circulant code (no reference
  * counterpart; results identical bit for bit).  On first use the plan
  * generates a decoder kernel with the code's layers, degrees, block columns
  * and shifts as constants and compiles it with NVRTC; min-sum decodes whose
  * frame groups have one thread per row slot (threads per frame == Z rounded
- * up to whole warps) then run it.  AUTO (the default) falls back to the
+ * up to whole warps) then run it, and sum-product decodes of small codes a
+ * program of their own (compiled on the first of them; without it, in every
+ * mode, the table-driven kernel serves).  AUTO (the default) falls back to the
  * table-driven kernel where NVRTC is missing or the environment sets
  * COMMKIT_GB300_SPECIALISE=0 (COMMKIT_GB300_NVRTC names the NVRTC library
  * to load instead of searching for it); ON makes an unavailable specialisation an
