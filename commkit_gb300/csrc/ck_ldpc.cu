@@ -69,13 +69,8 @@ template <int DMAX, template <bool> class State>
 struct MinSumPickOf {
     template <bool QC, bool ONE_ROW>
     static KernelFn get(bool app_smem, bool r_smem) {
-        // Codes without circulants and up to kPackedDegree edges per row run
-        // here only where decode_ell_kernel does not take them, which leaves
-        // no posterior small enough for shared memory.
-        if constexpr (QC || DMAX == 0) {
-            if (app_smem && r_smem) return decode_kernel<State, QC, DMAX, true, true, ONE_ROW>;
-            if (app_smem) return decode_kernel<State, QC, DMAX, true, false, ONE_ROW>;
-        }
+        if (app_smem && r_smem) return decode_kernel<State, QC, DMAX, true, true, ONE_ROW>;
+        if (app_smem) return decode_kernel<State, QC, DMAX, true, false, ONE_ROW>;
         if constexpr (!QC) return decode_kernel<State, QC, DMAX, false, false, false>;
         return nullptr;
     }
