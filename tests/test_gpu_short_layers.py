@@ -70,3 +70,11 @@ CASES = [(32400, 16200, 3, 2), (30000, 15000, 2, 155), (20000, 16200, 5, 1), (32
 @pytest.mark.parametrize("placement", [0, 1, 2])
 def test_posterior_in_shared_memory_without_row_groups(N, m, weight, frames, placement):
     check_serial(N, m, weight, frames, placement)
+
+
+# Layers of one row whose 32-row groups would fit: 32 times the rows' state.
+@pytest.mark.parametrize("N,m,weight,frames", [(16200, 9000, 3, 3), (2000, 1000, 3, 40), (600, 66, 2, 300)])
+@pytest.mark.parametrize("placement", [0, 2])
+def test_state_is_that_of_the_rows(N, m, weight, frames, placement):
+    _, need = check_serial(N, m, weight, frames, placement)
+    assert need <= 512 + frames * 2 * 12 * (m + 32)
