@@ -134,6 +134,7 @@ struct Resolved {
     int32_t sign_words;  // wide min-sum state: sign words per row (0: packed or sum-product)
     bool edges;  // min-sum with one message per edge in shared memory (CK_LDPC_PLACE_EDGES)
     bool ell;    // decode_ell_kernel
+    int ell_single;  // most frames that an SM takes as one-frame blocks of it (0: none)
     // The register form of a code that has one (null: none): its threads per frame, shared memory and blocks per SM.
     const void* reg_kernel;
     int32_t reg_T;
@@ -247,14 +248,13 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
         // same bits.
         const int64_t blocks = int64_t(sms) * per_sm;
         const int32_t g2 = static_cast<int32_t>((B + blocks - 1) / blocks);
-        if (r->ell && plan->launch.threads_per_frame == 0 && plan->launch.frames_per_block == 0) {
-            // One frame per block, its threads the share of an SM that the
-            // frames spread over all SMs leave each (the SMs hold them all:
-            // their shared memory does, and so do those threads).
-            r->T = std::max(r->T, ell_threads(plan, static_cast<int32_t>((B + sms - 1) / sms)));
+        const int64_t per = (B + sms - 1) / sms;  // frames per SM, spread over all SMs
+        if (per <= r->ell_single) {
+            // One frame per block, its threads the share of an SM that the frames on it leave each.
+            r->T = std::max(r->T, ell_threads(plan, static_cast<int32_t>(per)));
             G = r->G = 1;
             r->smem = r->tables_bytes + r->group_bytes;
-            per_sm = static_cast<int>((B + sms - 1) / sms);
+            per_sm = static_cast<int>(per);
         } else if (g2 >= 1 && g2 < G) {
             G = g2;
             r->G = g2;
@@ -480,6 +480,17 @@ int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_
     r->cluster_per_sm = 0;
     r->cluster = 1;
     r->ell = ell;
+    r->ell_single = 0;
+    if (ell && plan->launch.threads_per_frame == 0 && plan->launch.frames_per_block == 0) {
+        // As many as are resident at once with the threads that each then has: every such block has its own tables
+        // and the system's 1 KB.  4 iterations of N = 28500, of which one block holds two and an SM one block:
+        // 300 frames 201 us as single blocks, 157 in pairs; N = 2000, 2000 frames 182 and 157; N = 1000 144 and 70.
+        for (int f = 1, blocks = 1; blocks >= f; ++f) {
+            CK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, std::max(T, ell_threads(plan, f)),
+                                                                  tables + group));
+            if (blocks >= f) r->ell_single = f;
+        }
+    }
     r->reg_kernel = nullptr;
     if ((sp || (edge_kernel && plan->launch.frames_per_block == 0)) && plan->launch.threads_per_frame == 0 &&
         register_threads(*plan) > 0) {

@@ -45,6 +45,28 @@ CASES = [
 ]
 
 
+def test_short_batch_in_blocks_that_are_resident():
+    """A code of which a block holds two frames and an SM one block: a batch
+    of two frames per SM runs as blocks of two."""
+    import torch
+
+    import commkit_gb300 as ck
+
+    code = staircase_code(ck, 28500, 14250, 3, seed=4)
+    plan = code._plan(0)
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("frame counts of 152 SMs")
+    assert plan.workspace_size(301) == plan.workspace_size(302) > plan.workspace_size(300)
+    llrs = (1.5 + 2.0 * np.random.default_rng(2).standard_normal((301, code.n))).astype(np.float32)
+    row_ptr, cols, _ = code._schedule
+    method = ck.MinSum(max_iterations=3)
+    r = ck.decode(torch.from_numpy(llrs).cuda(), code=code, method=method)
+    want = oracle.decode(llrs, (row_ptr, cols, 28500), k=code.k, scale=method.scale, offset=method.offset,
+                         max_iterations=3, early_stop=True)  # fmt: skip
+    for g, w in zip((r.bits, r.llrs, r.valid, r.iterations), want, strict=True):
+        np.testing.assert_array_equal(g.cpu().numpy().reshape(w.shape), w)
+
+
 @pytest.mark.parametrize("N,m,weight,punctured,frames", CASES)
 @pytest.mark.parametrize("placement", [1, 2])
 def test_staircase_codes_equal_oracle(N, m, weight, punctured, frames, placement):
