@@ -203,6 +203,12 @@ void make_ell(const int32_t* row_ptr, const int32_t* cols, const int32_t* layer_
               ck_ldpc_plan* plan) {
     const int32_t L = plan->L, N = plan->N;
     if (plan->max_deg > ck::ldpc::kPackedDegree || N > 65535) return;  // places up to N in 16 bits
+    // Short codes with rows of up to 8 edges: the CSR rows, of 32 frames per block, are as fast or faster in batches
+    // (4 iterations, CSR rows against this form, 1 / 1000 / 5000 frames: N = 130 25 / 27 / 52 against 30 / 53 / 65
+    // us, N = 2000 35 / 70 / 233 against 32 / 83 / 242, N = 4000 38 / 102 / 403 against 37 / 114 / 454, N = 5000
+    // 52 / 151 / 577 against 37 / 134 / 551).  Longer rows gain at every length (N = 1000, rows of 13: 84 / 93 / 184
+    // against 42 / 50 / 135).
+    if (plan->max_deg <= 8 && N < 5000) return;
     // Layers are filled up to 32 rows, in the message state and the syndrome test as well: above twice the rows the
     // state outgrows the gain (N = 16200, 400 frames, 4 iterations, layers of 16 / 8 / 4 rows: 78 / 156 / 312 MB of
     // state against 39, and 1.28 / 4.9 / 10.1 ms against the CSR rows' 1.80 / 3.5 / 6.5).

@@ -78,3 +78,17 @@ def test_posterior_in_shared_memory_without_row_groups(N, m, weight, frames, pla
 def test_state_is_that_of_the_rows(N, m, weight, frames, placement):
     _, need = check_serial(N, m, weight, frames, placement)
     assert need <= 512 + frames * 2 * 12 * (m + 32)
+
+
+@pytest.mark.parametrize("N,m,weight,threads", [(130, 66, 2, 1024), (4999, 2500, 3, 1024), (5000, 2500, 3, 768), (1000, 250, 3, 512)])
+def test_short_codes_take_the_csr_rows(N, m, weight, threads):
+    """Rows of up to 8 edges below N = 5000 run the CSR rows (up to 1024
+    threads per frame; the 32-row groups cut a set shape to theirs)."""
+    import commkit_gb300 as ck
+
+    row_ptr, cols = staircase_rows(N, m, weight, seed=1)
+    checks = np.repeat(np.arange(m, dtype=np.int32), np.diff(row_ptr))
+    plan = ck.LDPCCode(checks, cols, m, N)._plan(0)
+    assert plan.info["quasi_cyclic"] == 0
+    plan.set_launch(1024, 0, 0)
+    assert plan.resolved_launch()[0] == threads
