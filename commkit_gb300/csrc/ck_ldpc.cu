@@ -145,7 +145,24 @@ struct Resolved {
 
 constexpr int kMaxCluster = 8;  // the portable cluster size
 constexpr uint32_t kRegAppOffset = 128;  // the posterior's place in the register form's shared memory
-constexpr int kRegWaves = 8;             // most min-sum waves it takes (ck_ldpc_regs.cuh has the figures)
+
+// Most waves of blocks that a min-sum batch takes in the register form.  It
+// holds fewer frames per SM than the shared form, so past its first wave it
+// wins by its rows' cost: two lanes per row fill the warps of short liftings
+// (below 17 the shared form's are half empty) and their joins count for less
+// in long rows; wide blocks leave an SM with 10 to 16 warps.  Shared form over
+// register form, frames stopping early, at 1 / 2 / 4 / 6 waves: Z = 16 with
+// rows of 5 1.65 / 1.56 / 1.55 / 1.52, code A (Z = 54, rows of 6.4) 1.39 / 1.11
+// / 1.01 / 0.98, Z = 27 with rows of 5 1.23 / 1.14 / 1.01 / 0.93, code B (Z = 96,
+// rows of 11) 1.16 / 1.07 / 1.06 / 1.03, Z = 160 with rows of 14 1.43 / 1.23 /
+// 1.04 / 1.07 (no early stop: 1.48 / 1.05 / 0.91 / 1.02) and of 6 1.20 / 0.98 /
+// 0.81 / 0.80, Z = 256 with rows of 5 0.98 / 0.89 / 0.86 / 0.75.
+int reg_waves(const ck_ldpc_plan* plan, int32_t threads) {
+    const int64_t rows = plan->m, edges = plan->E;
+    if (threads <= 32) return 8;
+    if (threads <= 224) return edges >= 6 * rows ? 8 : 4;
+    return edges >= 10 * rows ? 2 : 1;
+}
 
 constexpr size_t kHeaderBytes = 256;
 static_assert(4 * kMaxMixed <= kHeaderBytes, "the mixed launch's queue counters sit in the header");
@@ -228,10 +245,10 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
         }
     }
     // The register form (one frame per block): sum-product batches of every
-    // size, min-sum batches of up to kRegWaves waves, where the time of a
-    // frame counts for more than the frames an SM holds.
+    // size, min-sum batches of up to reg_waves, where the time of a frame
+    // counts for more than the frames an SM holds.
     const bool regs = r->reg_kernel && B > 0 &&
-                      (rule == CK_LDPC_SUM_PRODUCT || B <= int64_t(sms) * r->reg_per_sm * kRegWaves);
+                      (rule == CK_LDPC_SUM_PRODUCT || B <= int64_t(sms) * r->reg_per_sm * reg_waves(plan, r->reg_T));
     r->direct = regs && B <= int64_t(sms) * r->reg_per_sm;
     if (regs) {
         r->kernel = r->reg_kernel;

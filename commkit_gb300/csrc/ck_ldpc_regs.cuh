@@ -26,8 +26,8 @@ namespace ldpc {
 // Measured on code A (Z = 54, 124 registers, 4 frames per SM): 50 iterations
 // of 16 frames 113 to 64 us; with one message per edge in shared memory (10
 // frames per SM) 1024 frames at 2.5 dB 122 us against 88, 4096 183 against
-// 158, 8192 at 1.6 dB 447 against 483: batches of more than kRegWaves waves
-// keep the shared form.
+// 158, 8192 at 1.6 dB 447 against 483: batches of more waves
+// than reg_waves (ck_ldpc.cu) keep the shared form.
 //
 // Prog (generated): kSlots edge slots per lane;
 //   columns(a, a_addr, r, h, own)  the shared addresses of row r, half h;

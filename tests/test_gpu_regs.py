@@ -56,3 +56,48 @@ def test_circulant_codes_equal_oracle(mb, nb, z, weight, punctured, frames):
                 np.testing.assert_array_equal(g.cpu().numpy().reshape(w.shape), w, err_msg=what)
         wd = _device.wrap(ws)
         assert _lib.lib().ck_ldpc_workspace_status(wd.ptr, _device.stream_of(wd)) == _lib.CK_OK
+
+
+def _kernels(f):
+    """Names of the kernels that ``f`` launches, as the profiler sees them."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    f()
+    for _ in range(2):  # a process's first profile may come back empty
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            f()
+            torch.cuda.synchronize()
+    return {e.name for e in p.events()}
+
+
+# Information column weights 3 of 12 of 24 base columns (rows of 4.9) and 4 of 18 (13.8): short and long rows.
+@pytest.mark.parametrize("mb,z,weight,waves,beyond", [
+    (12, 160, 3, 1.0, 1.3),
+    (12, 256, 3, 1.0, 1.3),
+    (6, 160, 4, 2.0, 2.3),
+    (12, 54, 3, 4.0, 4.3),
+    (6, 64, 4, 8.0, 8.3),
+    (12, 16, 3, 8.0, 8.3),
+])  # fmt: skip
+def test_form_by_waves(mb, z, weight, waves, beyond):
+    """The register form up to the waves that its width and row length bear,
+    the shared form beyond (both bit-identical)."""
+    import torch
+
+    import commkit_gb300 as ck
+
+    base = W.dual_diagonal_base(mb, 24, z, (weight,) * (24 - mb), seed=z)
+    code = ck.LDPCCode.quasi_cyclic(base, lifting=z)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    slots = sum((int(d) + 1) // 2 for d in (base >= 0).sum(1))
+    threads = (z + 15) // 16 * 32
+    per_sm = min(max(65536 // ((2 * slots + 40 + 7) // 8 * 8 * threads), 1), 16)
+    names = {}
+    for w in (waves, beyond):
+        x = torch.full((int(w * sms * per_sm), code.n), 4.0, device="cuda")
+        names[w] = _kernels(lambda: ck.decode(x, code=code, method=ck.MinSum(max_iterations=2)))
+    if not any(k.startswith("ck_ldpc") for n in names.values() for k in n):
+        pytest.skip("no profiler")
+    assert "ck_ldpc_code_r3" in names[waves] and "ck_ldpc_code_r3" not in names[beyond]
