@@ -468,6 +468,7 @@ class _Plan:
         """``_lib.CK_LDPC_SPECIALISE_{AUTO,OFF,ON}``: whether decodes of
         this circulant code run its code-specialised kernels."""
         _lib.check(_lib.lib().ck_ldpc_plan_set_specialise(self.handle, int(mode)), "set_specialise")
+        self.__dict__.pop("_ws_need", None)  # the forms differ in their device-memory state
 
     def specialisation(self) -> tuple[int, int, str]:
         """(mode, state, reason): state 1 compiled, 0 not yet, -1 unavailable

@@ -256,6 +256,7 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
         G = r->G = 1;
         r->smem = r->reg_smem;
         r->app_off = kRegAppOffset;
+        r->r_slot_bytes = r->app_slot_bytes = 0;  // the table-driven kernel's, which this form has no use for
         per_sm = r->reg_per_sm;
     }
     if (!regs && r->cluster <= 1 && B > 0 && B < int64_t(sms) * per_sm * G) {

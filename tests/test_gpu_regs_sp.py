@@ -64,3 +64,31 @@ def test_row_of_two_edges():
     base = W.dual_diagonal_base(6, 12, 17, (3,) * 6, seed=1)
     base[4, :6] = -1
     _run(base, 17, 40)
+
+
+def test_no_workspace_for_messages_in_registers():
+    """The register form keeps nothing in device memory, also for a code
+    whose messages the table-driven kernel keeps there; a plan whose
+    specialisation is turned off asks for that kernel's workspace anew."""
+    import torch
+
+    import commkit_gb300 as ck
+    from commkit_gb300 import _lib
+
+    rng = np.random.default_rng(8)
+    base = np.full((8, 40), -1, np.int64)  # rows of 16: 64 edge slots per lane, 25,600 messages
+    for i in range(8):
+        base[i, (5 * i + np.arange(16)) % 40] = rng.integers(0, 200, 16)
+    code = ck.LDPCCode.quasi_cyclic(base, lifting=200)
+    plan = code._plan(0)
+    assert plan.workspace_size(300, _lib.CK_LDPC_SUM_PRODUCT) <= 512
+    x = torch.from_numpy((1.5 + 1.7 * rng.standard_normal((300, code.n))).astype(np.float32)).cuda()
+    method = ck.SumProduct(max_iterations=4)
+    ws = torch.full((512,), 255, dtype=torch.uint8, device="cuda")
+    got = [ck.decode(x, code=code, method=method), ck.decode(x, code=code, method=method, workspace=ws)]
+    plan.set_specialise(_lib.CK_LDPC_SPECIALISE_OFF)
+    assert plan.workspace_size(300, _lib.CK_LDPC_SUM_PRODUCT) >= 152 * 4 * 25600
+    want = ck.decode(x, code=code, method=method)
+    for g in got:
+        for name in ("bits", "llrs", "valid", "iterations"):
+            np.testing.assert_array_equal(getattr(g, name).cpu().numpy(), getattr(want, name).cpu().numpy(), err_msg=name)
