@@ -18,8 +18,8 @@
 // four rows per thread, whose column loads are in flight together, each chunk
 // scanned over its chains in shared memory.  Measured (encode_blocks): 1000 frames
 // of code C 130 to 31 us, 4096 frames of code A 31 to 14 us (the launch), 128
-// frames of DVB-S2 normal 97 to 64 us; one frame of the latter 50 to 62 us,
-// a single block's chain of 32400 rows.
+// frames of DVB-S2 normal 97 to 64 us.  A few frames of one long chain
+// keep the byte-wise kernels (few_long_frames, ck_sim.cu).
 #include <stdint.h>
 
 #include <algorithm>

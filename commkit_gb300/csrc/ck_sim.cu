@@ -17,9 +17,9 @@
 //
 // Every kernel is a plain grid over its outputs with bounds checks.  The
 // accumulator encoder is ck_ldpc_encode.cu; the encoding kernels here serve a
-// GF(2) inverse, a systematic generator, and accumulators whose information
-// bits exceed a block's shared memory (long chains by one block-wide XOR scan
-// per chain).
+// GF(2) inverse, a systematic generator, a few frames of one long chain, and
+// accumulators whose information bits exceed a block's shared memory (long
+// chains by one block-wide XOR scan per chain).
 #include <stdint.h>
 
 #include "ck_common.cuh"
@@ -423,6 +423,24 @@ extern "C" int ck_random_bits(int8_t* out, int64_t count, uint64_t seed, uint64_
     return ck::cuda_check(cudaGetLastError(), "random bits launch");
 }
 
+namespace {
+
+// An accumulator of one chain is one block per group of frames in
+// ck_ldpc_encode.cu, which packs all k bits and walks all m rows by itself:
+// a few frames of a long code leave the GPU idle.  The byte-wise kernels
+// spread both over it, for three launches (17 us in a row) and a chain of 1.5
+// us per 1000 rows.  Byte-wise against one block, (k, m): (48600, 16200) 1 /
+// 32 / 64 / 152 frames 31 / 43 / 53 / 86 against 69 / 69 / 69 / 71 us, (32400,
+// 32400) 50 / 64 / 74 / 111 against 63 / 64 / 65 / 65, (25920, 38880) 59 / 69 / 77
+// / 112 against 60, (7200, 9000) 18 / 21 / 24 / 32 against 25, (9000, 3000) 17
+// against 15, (3000, 3000) 18 against 13.
+bool few_long_frames(int64_t B, int32_t k, int32_t m, int32_t g) {
+    return g == 1 && static_cast<int64_t>(k) + m >= 14000 && 4 * static_cast<int64_t>(m) <= 5 * static_cast<int64_t>(k) &&
+           B <= 64 && B * m <= 40 * static_cast<int64_t>(k);
+}
+
+}  // namespace
+
 extern "C" int ck_ldpc_encode(const int8_t* info, int64_t B, int32_t k, int32_t m, int32_t n,
                               const int32_t* info_row_ptr, const int32_t* info_cols, int32_t stride,
                               const uint32_t* inverse, int8_t* scratch, size_t scratch_bytes,
@@ -441,13 +459,13 @@ extern "C" int ck_ldpc_encode(const int8_t* info, int64_t B, int32_t k, int32_t 
     if (scratch_bytes < need)
         return ck::fail(CK_ERR_INVALID_ARGUMENT, "scratch of %zu bytes, %zu needed", scratch_bytes, need);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!inverse) {
+    if (!inverse && !few_long_frames(B, k, m, stride)) {
         bool done = false;
         CK_TRY(ck::encode_accumulate(info, B, k, m, n, info_row_ptr, info_cols, stride, words, nullptr, st, &done));
         if (done) return CK_OK;
     }
-    // A GF(2) inverse, or an accumulator whose information bits exceed a
-    // block's shared memory.
+    // A GF(2) inverse, a few frames of one long chain, or an accumulator whose
+    // information bits exceed a block's shared memory.
     copy_info_kernel<<<grid_for(static_cast<uint64_t>(B) * k), kThreads, 0, st>>>(info, B, k, n, words);
     syndrome_kernel<<<grid_for(static_cast<uint64_t>(B) * m), kThreads, 0, st>>>(info, B, k, m, info_row_ptr,
                                                                                   info_cols, scratch);

@@ -80,3 +80,34 @@ def test_accumulator_codes_equal_host(k, m, g, punctured, frames):
         y[frames - 1, k - 1] = bad
         with pytest.raises(ValueError, match="0 or 1"):
             ck.encode(y, code=code)
+
+
+# k, m, frames on both sides of the line between the byte-wise kernels and the one-kernel encoder.
+@pytest.mark.parametrize("k,m,frames,few", [
+    (9000, 5000, 1, True),
+    (9000, 5000, 64, True),
+    (9000, 5000, 65, False),
+    (7200, 9000, 32, True),
+    (7200, 9000, 33, False),
+    (9000, 4999, 1, False),
+    (6200, 7800, 1, False),
+])  # fmt: skip
+def test_few_frames_of_a_long_chain(k, m, frames, few):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    import commkit_gb300 as ck
+    from commkit_gb300.coding import encode_blocks
+
+    code = accumulator_code(ck, k, m, 1, 0, seed=k + m)
+    info = np.random.default_rng(5).integers(0, 2, (frames, k), dtype=np.int8)
+    x = torch.from_numpy(info).cuda()
+    np.testing.assert_array_equal(encode_blocks(code, x).cpu().numpy(), host_encode(code, 1, info))
+    for _ in range(2):  # a process's first profile may come back empty
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            encode_blocks(code, x)
+            torch.cuda.synchronize()
+    names = " ".join(e.name for e in p.events())
+    if "_kernel" not in names:
+        pytest.skip("no profiler")
+    assert ("syndrome_kernel" in names) == few and ("encode_kernel" in names) != few
