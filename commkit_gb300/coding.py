@@ -811,6 +811,12 @@ def _encode_rows(code: LDPCCode, like: _device.DeviceArray, info: int, R: int, w
     _lib.check(st, "encode()")
 
 
+# The most information bits that the checking encoder's block can hold: a word
+# each beside 34 KB of packing tiles and a word per residue in 227 KB (near it
+# the C call may still refuse a wide accumulator).
+_MAX_CHECKED = 49376
+
+
 def _encode_checked(bits: Any, x: _device.DeviceArray, code: LDPCCode) -> Any:
     """:func:`encode` of int8 or uint8 torch bits by an accumulator: one
     kernel reads the bits, checks them and writes the codewords (the checks
@@ -821,7 +827,7 @@ def _encode_checked(bits: Any, x: _device.DeviceArray, code: LDPCCode) -> Any:
         return None
     e = code._encoder
     k, n = code.k, code.n
-    if e.inverse is not None or e.generator is not None or x.shape[-1] % k:
+    if e.inverse is not None or e.generator is not None or x.shape[-1] % k or k > _MAX_CHECKED:
         return None
     import torch
 

@@ -111,3 +111,24 @@ def test_few_frames_of_a_long_chain(k, m, frames, few):
     if "_kernel" not in names:
         pytest.skip("no profiler")
     assert ("syndrome_kernel" in names) == few and ("encode_kernel" in names) != few
+
+
+def test_more_bits_than_a_block_holds_go_straight_to_the_general_path(monkeypatch):
+    """encode() allocates and calls nothing for the checking kernel where it
+    cannot serve; just below, it serves."""
+    import torch
+
+    import commkit_gb300 as ck
+    from commkit_gb300 import _lib
+
+    lib = _lib.lib()
+    calls = []
+    checked = lib.ck_ldpc_encode_checked
+    monkeypatch.setattr(lib, "ck_ldpc_encode_checked", lambda *a: (calls.append(a[2]), checked(*a))[1])
+    for k, served in ((49376, True), (49377, False)):
+        code = accumulator_code(ck, k, 600, 1, 0, seed=k)
+        info = np.random.default_rng(6).integers(0, 2, (2, k), dtype=np.int8)
+        calls.clear()
+        got = ck.encode(torch.from_numpy(info).cuda(), code=code)
+        np.testing.assert_array_equal(got.cpu().numpy(), host_encode(code, 1, info))
+        assert (len(calls) == 1) == served
