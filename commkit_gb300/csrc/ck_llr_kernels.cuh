@@ -84,8 +84,8 @@ struct LevelAxis {
     // then the halves of every bit are known at compile time.
     alignas(16) float2 lp[L];
     int32_t gray;
-    // Each level, and its log prior times log2(e), twice, as the two-symbol
-    // steps read them, and whether any log prior is not 0.
+    // Each level, and its log prior, twice, as the two-symbol steps read them,
+    // and whether any log prior is not 0.
     alignas(16) float2 lev2[L], lp2[L];
     int32_t priors;
     alignas(8) float nz[2];  // (-0, -0): the addend of the two-lane products (mul2z)
@@ -463,7 +463,8 @@ __device__ __forceinline__ uint64_t log2_of2(uint64_t x) {
 
 // Noise scale of the two-symbol steps: -log2(e)/sigma^2 and its negative
 // rounded to float, and ln 2 corrected for that rounding (the LLR is the
-// base-2 one times hi + lo).
+// base-2 one times hi + lo).  With priors (natural) the scale stays 1/sigma^2,
+// which a log prior meets unrounded, and ln 2 is itself.
 struct PairScale {
     uint64_t neg, pos, lo;
     static __device__ __forceinline__ void one(float s2, float& s, float& lo) {
@@ -473,6 +474,14 @@ struct PairScale {
         // s = s2 log2(e) (1 + eps); below 1e-30 (LLRs of 0) eps could not be formed.
         const float r = __fmaf_rn(s2, kL2ELo, __fmaf_rn(s2, kL2E, -s));
         lo = s >= 1e-30f ? __fmaf_rn(__fmul_rn(r, 0.6931471824645996f), __frcp_rn(s), kLn2Lo) : kLn2Lo;
+    }
+    __device__ __forceinline__ PairScale() {}
+    static __device__ __forceinline__ PairScale natural(float sa, float sb) {
+        PairScale r;
+        r.pos = pk2(sa, sb);
+        r.neg = pk2(-sa, -sb);
+        r.lo = pk2(-1.904654290582768e-9f, -1.904654290582768e-9f);
+        return r;
     }
     __device__ __forceinline__ PairScale(float sa, float sb) {
         float a, b, la, lb;
@@ -484,12 +493,20 @@ struct PairScale {
     }
 };
 
+__device__ __forceinline__ uint64_t log2e2() { return pk2(1.44269502162933349609375f, 1.44269502162933349609375f); }
+// e^x, with what the rounding of x log2(e) left out.
+__device__ __forceinline__ uint64_t exp_natural2(uint64_t x) {
+    const uint64_t y = mul2(x, log2e2()), e = ex2_of2(y);
+    return fma2(e, fma2(y, pk2(-0.6931471824645996f, -0.6931471824645996f), x), e);
+}
+
 // log2 of a half-sum (bit b >= 1, half v) whose terms underflow beside the
 // symbol's peak: relative to the half's own nearest level, over its levels
-// only, then shifted to the peak's scale (np: the peak's scaled distance).
+// only, then shifted to the peak's scale (np: the peak's scaled distance);
+// with priors the shift goes to `shift`, natural.
 template <int KA, bool PRIORS>
 __device__ __forceinline__ uint64_t half_log2(uint64_t x, const LevelAxis<KA>& t, const PairScale& s, uint64_t np,
-                                              uint64_t nz, int b, int v) {
+                                              uint64_t nz, int b, int v, uint64_t& shift) {
     constexpr int L = 1 << KA;
     uint64_t d2[L];
     float na = ck::inf_f(), nb = ck::inf_f();
@@ -514,9 +531,13 @@ __device__ __forceinline__ uint64_t half_log2(uint64_t x, const LevelAxis<KA>& t
 #pragma unroll
     for (int j = 0; j < L; ++j) {
         if (gray_bit<KA>(j, b) != v) continue;
-        const uint64_t e = ex2_of2(PRIORS ? sub2(p, d2[j]) : fma2(d2[j], s.neg, p));
+        const uint64_t e = PRIORS ? exp_natural2(sub2(p, d2[j])) : ex2_of2(fma2(d2[j], s.neg, p));
         sum = first ? e : add2(sum, e);
         first = false;
+    }
+    if constexpr (PRIORS) {
+        shift = sub2(np, p);
+        return log2_of2(sum);
     }
     return add2(log2_of2(sum), sub2(np, p));
 }
@@ -524,15 +545,17 @@ __device__ __forceinline__ uint64_t half_log2(uint64_t x, const LevelAxis<KA>& t
 // Exact base-2 LLRs of one axis for two symbols at once (x: their
 // coordinates), Gray labels: o[b] for b >= 1; the first bit's is
 // np[1] - np[0] + o[0], its halves' nearest levels and the rest (first_bit
-// joins them).  What bounds this method is issue
+// joins them); with priors plus shift[b], natural.  What bounds this method is issue
 // (417 instructions per 64-QAM symbol one level at a time) and then the
 // hardware's 2^x and log2 units, so:
 //  * the two symbols are the lanes of the two-lane forms throughout, and the
 //    metrics are in base 2 (PairScale), which takes the logs' and
 //    exponentials' factors out: a level costs two operations for its squared
 //    distance, one fused multiply-add for its exponent (one rounding less
-//    than metric and difference) and one 2^x; with priors (PRIORS) the
-//    scaled distance less the level's prior is formed first;
+//    than metric and difference) and one 2^x.  With priors (PRIORS) the
+//    scaled distance less the level's prior is formed first, in the natural
+//    scale, in one rounding, and the difference to the nearest one goes to
+//    base 2: a log prior times log2(e) would be rounded beside it;
 //  * the exponents are relative to the nearest level of each half of the
 //    axis, not of the whole: the first bit's two sums (its halves are these)
 //    never underflow, whatever the SNR, and the other bits' sums join the
@@ -543,10 +566,14 @@ __device__ __forceinline__ uint64_t half_log2(uint64_t x, const LevelAxis<KA>& t
 // on this axis are the level-by-level method's.
 // Measured against that method, 2^22 symbols: 4 / 16 / 64 / 256-QAM at 11 /
 // 11 / 18.6 / 24 dB 21 / 34 / 76 / 185 -> 13 / 25 / 36 / 82 us (2.0 to 5.4
-// TB/s), shaped 64-QAM 99 -> 52 us, with no more error against 64 bits.
+// TB/s), with no more error against 64 bits.  Shaped 16 / 64 / 256-QAM at 15 /
+// 20 / 25 dB 62 / 122 / 266 -> 39 / 77 / 150 us; root mean square errors over
+// 0 to 32 dB 0.94 to 0.99 times that method's (in base 2, with the priors'
+// products rounded, 31 / 63 / 118 us and up to 1.09 times, 1.3 at single
+// points).
 template <int KA, bool PRIORS>
 __device__ __forceinline__ int axis_exact_pair(uint64_t x, const LevelAxis<KA>& t, const PairScale& s,
-                                               uint64_t nz, uint64_t (&np)[2], uint64_t* o) {
+                                               uint64_t nz, uint64_t (&np)[2], uint64_t* o, uint64_t* shift) {
     constexpr int L = 1 << KA, H = L / 2;
     const uint32_t base = ck::smem_addr(&t.lev2[0]);
     uint64_t d2[L];
@@ -580,7 +607,8 @@ __device__ __forceinline__ int axis_exact_pair(uint64_t x, const LevelAxis<KA>& 
     if constexpr (KA > 1) {
         uint64_t e[L];
 #pragma unroll
-        for (int j = 0; j < L; ++j) e[j] = ex2_of2(PRIORS ? sub2(np[j / H], d2[j]) : fma2(d2[j], s.neg, np[j / H]));
+        for (int j = 0; j < L; ++j)
+            e[j] = PRIORS ? exp_natural2(sub2(np[j / H], d2[j])) : ex2_of2(fma2(d2[j], s.neg, np[j / H]));
         // Sums of each half, and of its levels whose bit b is v (bit b < KA - 1
         // is constant on pairs of levels, the last one on pairs' neighbours),
         // each from the outside in, so that a tie gives equal sums.
@@ -616,7 +644,13 @@ __device__ __forceinline__ int axis_exact_pair(uint64_t x, const LevelAxis<KA>& 
         // Weights of the halves beside the symbol's peak: 1 and 2^-|diff|.
         float da, db;
         upk2(diff, da, db);
-        const float wa = ex2_of(-fabsf(da)), wb = ex2_of(-fabsf(db));
+        float wa, wb;
+        if constexpr (PRIORS) {
+            upk2(exp_natural2(pk2(-fabsf(da), -fabsf(db))), wa, wb);
+        } else {
+            wa = ex2_of(-fabsf(da));
+            wb = ex2_of(-fabsf(db));
+        }
         const uint64_t w0 = pk2(da < 0.0f ? wa : 1.0f, db < 0.0f ? wb : 1.0f);
         const uint64_t w1 = pk2(da < 0.0f ? 1.0f : wa, db < 0.0f ? 1.0f : wb);
         float low_a = 1.0f, low_b = 1.0f;
@@ -636,7 +670,8 @@ __device__ __forceinline__ int axis_exact_pair(uint64_t x, const LevelAxis<KA>& 
         for (int b = 1; b < KA; ++b)
 #pragma unroll
             for (int v = 0; v < 2; ++v) lg[b][v] = log2_of2(sum[b][v]);
-        constexpr float kFloor = 7.8886090522101181e-31f;  // 2^-100
+        // 2^-100; with priors the level-by-level method's: log2's error grows with the log, half_log2's does not.
+        constexpr float kFloor = PRIORS ? kExactFloor : 7.8886090522101181e-31f;
         if (!(fminf(low_a, low_b) >= kFloor)) {
             float p0a, p0b, p1a, p1b;
             upk2(np[0], p0a, p0b);
@@ -650,8 +685,14 @@ __device__ __forceinline__ int axis_exact_pair(uint64_t x, const LevelAxis<KA>& 
                     upk2(sum[b][v], ma, mb);
                     if (fminf(ma, mb) >= kFloor) continue;
                     upk2(lg[b][v], la, lb);
-                    upk2(half_log2<KA, PRIORS>(x, t, s, peak, nz, b, v), ra, rb);
+                    uint64_t by = 0ull;
+                    upk2(half_log2<KA, PRIORS>(x, t, s, peak, nz, b, v, by), ra, rb);
                     lg[b][v] = pk2(ma >= kFloor ? la : ra, mb >= kFloor ? lb : rb);
+                    if constexpr (PRIORS) {
+                        upk2(by, ra, rb);
+                        by = pk2(ma >= kFloor ? 0.0f : ra, mb >= kFloor ? 0.0f : rb);
+                        shift[b] = v ? sub2(shift[b], by) : add2(shift[b], by);
+                    }
                 }
         }
 #pragma unroll
@@ -698,6 +739,15 @@ __device__ __forceinline__ uint64_t first_bit(const uint64_t (&np)[2], uint64_t 
     return pk2(__uint_as_float(__float_as_uint(ra) ^ sa), __uint_as_float(__float_as_uint(rb) ^ sb));
 }
 
+// The same from natural distances: (np[1] - np[0]) and what its rounding left
+// out, then the rest times ln 2, in one last rounding.
+__device__ __forceinline__ uint64_t first_bit_natural(const uint64_t (&np)[2], uint64_t rest, uint64_t hi, uint64_t lo) {
+    const uint64_t diff = sub2(np[1], np[0]);
+    const uint64_t part = sub2(diff, np[1]);  // -np[0], as far as diff holds it
+    const uint64_t left = sub2(sub2(np[1], sub2(diff, part)), add2(np[0], part));
+    return add2(diff, add2(left, fma2(rest, hi, mul2(rest, lo))));
+}
+
 template <int KA>
 __device__ __forceinline__ void load_level_axis(LevelAxis<KA>& t, const ck_axis_levels& a) {
     constexpr int L = 1 << KA;
@@ -708,8 +758,7 @@ __device__ __forceinline__ void load_level_axis(LevelAxis<KA>& t, const ck_axis_
         constexpr int R = LevelAxis<KA>::R;
         t.lp[i] = make_float2(a.levels[i], a.logp[i]);
         t.lev2[i] = make_float2(a.levels[i], a.levels[i]);
-        const float lp = __fmul_rn(a.logp[i], 1.44269502162933349609375f);
-        t.lp2[i] = make_float2(lp, lp);
+        t.lp2[i] = make_float2(a.logp[i], a.logp[i]);
         t.rec[i][0] = a.levels[i];
         t.rec[i][1] = a.logp[i];
 #pragma unroll
@@ -819,15 +868,17 @@ struct Tables<KA, 2> : Tables<KA, 1> {  // level metrics, exact
         }
         const uint64_t nz = lds_nz(ck::smem_addr(&this->re.nz[0]));
         const uint64_t hi = pk2(0.6931471824645996f, 0.6931471824645996f);
-        uint64_t o[2 * KA], np[2][2];
-        const int off_re = axis_exact_pair<KA, PRIORS>(pk2(xa.x, xb.x), this->re, s, nz, np[0], o);
-        const int off_im = axis_exact_pair<KA, PRIORS>(pk2(xa.y, xb.y), this->im, s, nz, np[1], o + KA);
+        uint64_t o[2 * KA], np[2][2], shift[2 * KA];
+#pragma unroll
+        for (int b = 0; b < 2 * KA; ++b) shift[b] = 0ull;
+        const int off_re = axis_exact_pair<KA, PRIORS>(pk2(xa.x, xb.x), this->re, s, nz, np[0], o, shift);
+        const int off_im = axis_exact_pair<KA, PRIORS>(pk2(xa.y, xb.y), this->im, s, nz, np[1], o + KA, shift + KA);
 #pragma unroll
         for (int b = 0; b < 2 * KA; ++b) {
             if (b % KA == 0)
-                o[b] = first_bit(np[b / KA], o[b], hi, s.lo);
+                o[b] = PRIORS ? first_bit_natural(np[b / KA], o[b], hi, s.lo) : first_bit(np[b / KA], o[b], hi, s.lo);
             else
-                o[b] = fma2(o[b], hi, mul2(o[b], s.lo));
+                o[b] = fma2(o[b], hi, PRIORS ? fma2(o[b], s.lo, shift[b]) : mul2(o[b], s.lo));
             upk2(o[b], oa[b], ob[b]);
         }
         if (off_re | off_im) {  // rare
@@ -860,7 +911,7 @@ struct Tables<KA, 2> : Tables<KA, 1> {  // level metrics, exact
     __device__ __noinline__ void pair_call(float2 x, float s2, float* o) const {
         float same[2 * KA];
         if (priors())
-            pair<true>(x, x, PairScale(s2, s2), s2, s2, o, same);
+            pair<true>(x, x, PairScale::natural(s2, s2), s2, s2, o, same);
         else
             pair<false>(x, x, PairScale(s2, s2), s2, s2, o, same);
     }
@@ -955,24 +1006,30 @@ __global__ void __launch_bounds__(kThreads, llr_blocks(METHOD, KA)) llr_kernel(c
                 const float2 a = ld_stream(x + 2 * p), b = ld_stream(x + 2 * p + 1);
                 return make_float4(a.x, a.y, b.x, b.y);
             };
-            const PairScale one(noise.value, noise.value);
-            const bool priors = tab.priors();
-            float4 v = load(t0);
-            for (uint32_t p = t0; p < npairs; p += stride) {
-                const float4 w = load(p + stride);
-                float sa, sb;
-                noise.pair(2 * p, sa, sb);
-                float o[2 * K];
-                const PairScale ps = noise.frames ? PairScale(sa, sb) : one;
-                if (priors)
-                    tab.template pair<true>(make_float2(v.x, v.y), make_float2(v.z, v.w), ps, sa, sb, o, o + K);
-                else
-                    tab.template pair<false>(make_float2(v.x, v.y), make_float2(v.z, v.w), ps, sa, sb, o, o + K);
-                float4* dst = reinterpret_cast<float4*>(out + static_cast<uint64_t>(p) * 2 * K);
+            const auto pairs = [&](const auto& step) {
+                float4 v = load(t0);
+                for (uint32_t p = t0; p < npairs; p += stride) {
+                    const float4 w = load(p + stride);
+                    float sa, sb;
+                    noise.pair(2 * p, sa, sb);
+                    float o[2 * K];
+                    step(make_float2(v.x, v.y), make_float2(v.z, v.w), sa, sb, o);
+                    float4* dst = reinterpret_cast<float4*>(out + static_cast<uint64_t>(p) * 2 * K);
 #pragma unroll
-                for (int q = 0; q < K / 2; ++q)
-                    st_stream(dst + q, make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]));
-                v = w;
+                    for (int q = 0; q < K / 2; ++q)
+                        st_stream(dst + q, make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]));
+                    v = w;
+                }
+            };
+            if (tab.priors()) {
+                pairs([&](float2 xa, float2 xb, float sa, float sb, float* o) {
+                    tab.template pair<true>(xa, xb, PairScale::natural(sa, sb), sa, sb, o, o + K);
+                });
+            } else {
+                const PairScale one(noise.value, noise.value);
+                pairs([&](float2 xa, float2 xb, float sa, float sb, float* o) {
+                    tab.template pair<false>(xa, xb, noise.frames ? PairScale(sa, sb) : one, sa, sb, o, o + K);
+                });
             }
             if ((n & 1u) && t0 == 0) {
                 const uint32_t i = n - 1;

@@ -92,3 +92,32 @@ def test_frames_and_nonfinite(order):
     assert np.all(np.isfinite(got[[0, 3, 5]]))
     assert np.all(got[0, k // 2] == 0.0)  # on the axis: a tie
     assert np.all(np.isnan(got[[1, 2], : k // 2])) and np.all(np.isnan(got[4, k // 2 :]))
+
+
+def test_shaped_error_no_larger_than_level_by_level():
+    """With priors, the two-symbol steps' error against float64 is, over the
+    noise range, no larger than that of the level-by-level method, which the
+    same constellation takes with every label bit inverted (the same LLRs,
+    negated)."""
+    import torch
+
+    import commkit_gb300 as ck
+
+    for order, nu in ((16, 0.5), (16, 1.0), (64, 0.2), (64, 0.5), (64, 1.0), (256, 0.2), (256, 0.5)):
+        c = ck.Constellation.qam(order).shaped(nu=nu)
+        inverted = ck.Constellation(c.points, 1 - np.asarray(c.bit_labels), c.pmf)
+        assert inverted._axes is not None
+        rng = np.random.default_rng(order)
+        ratios = []
+        for esn0_db in range(0, 33, 4):
+            nv = 10.0 ** (-esn0_db / 10.0)
+            n = 20000
+            x = c.points[rng.choice(order, n, p=np.asarray(c.pmf) / np.sum(c.pmf))]
+            x = (x + np.sqrt(nv / 2) * (rng.standard_normal(n) + 1j * rng.standard_normal(n))).astype(np.complex64)
+            want, _ = exact64(x, c, np.full(n, float(np.float32(1.0 / nv))))
+            t = torch.from_numpy(x).cuda()
+            got = ck.compute_llr(t, noise_var=nv, constellation=c, method="exact").cpu().numpy()
+            levels = -ck.compute_llr(t, noise_var=nv, constellation=inverted, method="exact").cpu().numpy()
+            rms = [np.sqrt(np.mean((v.reshape(want.shape).astype(np.float64) - want) ** 2)) for v in (got, levels)]
+            ratios.append(rms[0] / rms[1])
+        assert np.mean(ratios) <= 1.0, (order, nu, ratios)
