@@ -78,15 +78,14 @@ struct ck_ldpc_plan {
     // use: one per message-state placement.
     struct Jit {
         bool tried = false;
-        int dmax = 0;
         cudaLibrary_t lib = nullptr;
-        const void* kernel[4] = {nullptr, nullptr, nullptr, nullptr};  // by placement: device, records, edges, registers
-        std::string why;  // why there are none
+        const void* kernel = nullptr;
+        std::string why;  // why there is none
     };
     uint64_t id = 0;  // unique in the process, never reused
     int32_t jit_mode = CK_LDPC_SPECIALISE_AUTO;
-    mutable Jit jit;
-    mutable Jit jit_sp;  // the sum-product register form, compiled on its first use
+    mutable Jit jit[4];  // by placement: device, records, edges, registers
+    mutable Jit jit_sp;  // the sum-product register form
     mutable std::mutex jit_mu;
 };
 

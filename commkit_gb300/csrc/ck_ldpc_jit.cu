@@ -417,18 +417,19 @@ std::string sum_product_source(const ck_ldpc_plan& plan) {
            registers_struct(plan, "RegisterProgram", true) + "}  // namespace\n" + registers_kernel(plan, "ck_ldpc_code_sp");
 }
 
-// The plain decoder of one code: one kernel per message-state placement
+// The plain decoder of one code, for one message-state placement or all:
 // (r0 records in device memory, r1 records in shared memory, r2 one
 // message per edge in shared memory, r3 in registers where the code has
 // that form).
-std::string program_source(const ck_ldpc_plan& plan, int dmax) {
-    const int32_t reg_threads = register_threads(plan);
+std::string program_source(const ck_ldpc_plan& plan, int dmax, int only = -1) {
+    const bool registers = register_threads(plan) > 0 && (only < 0 || only == kPlaceRegisters);
     std::string s = "#include \"ck_ldpc_regs.cuh\"\nusing namespace ck::ldpc;\nnamespace {\n";
-    s += program_struct(plan, "CodeProgram");
-    if (reg_threads) s += registers_struct(plan, "RegisterProgram", false);
+    if (only != kPlaceRegisters) s += program_struct(plan, "CodeProgram");
+    if (registers) s += registers_struct(plan, "RegisterProgram", false);
     s += "}  // namespace\n";
-    if (reg_threads) s += registers_kernel(plan, "ck_ldpc_code_r3");
+    if (registers) s += registers_kernel(plan, "ck_ldpc_code_r3");
     for (int r = 0; r < 3; ++r) {
+        if (only >= 0 && r != only) continue;
         // A minimum of one block per SM, stated: without it ptxas held some of
         // these kernels to 40 registers and spilled.
         add(s, "extern \"C\" __global__ void __launch_bounds__(%lld, 1) ck_ldpc_code_r%lld(const __grid_constant__ Params p) {\n",
@@ -583,13 +584,13 @@ int specialised_kernel(const ck_ldpc_plan* plan, int dmax, int place, const void
     const int mode = effective_mode(plan->jit_mode);
     if (mode == CK_LDPC_SPECIALISE_OFF) return CK_OK;
     std::lock_guard<std::mutex> lock(plan->jit_mu);
-    ck_ldpc_plan::Jit& j = plan->jit;
+    ck_ldpc_plan::Jit& j = plan->jit[place];
     if (!j.tried) {  // a plan's degree bound never changes, so one compilation serves it
+        // One kernel at a time: a plan runs one placement, and the register
+        // form beside it, of the four.
         j.tried = true;
-        j.dmax = dmax;
         static const char* const names[] = {"ck_ldpc_code_r0", "ck_ldpc_code_r1", "ck_ldpc_code_r2", "ck_ldpc_code_r3"};
-        if (!compile_load(program_source(*plan, dmax), plan->device, names, register_threads(*plan) ? 4 : 3, &j.lib,
-                          j.kernel, &j.why))
+        if (!compile_load(program_source(*plan, dmax, place), plan->device, names + place, 1, &j.lib, &j.kernel, &j.why))
             j.lib = nullptr;
     }
     if (!j.lib) {
@@ -597,7 +598,7 @@ int specialised_kernel(const ck_ldpc_plan* plan, int dmax, int place, const void
             return ck::fail(CK_ERR_UNSUPPORTED, "code-specialised decoder unavailable: %s", j.why.c_str());
         return CK_OK;
     }
-    *out = j.kernel[place];
+    *out = j.kernel;
     return CK_OK;
 }
 
@@ -608,9 +609,9 @@ const void* sum_product_register_kernel(const ck_ldpc_plan* plan, bool may_compi
     if (!j.tried && may_compile) {
         j.tried = true;
         static const char* const names[] = {"ck_ldpc_code_sp"};
-        if (!compile_load(sum_product_source(*plan), plan->device, names, 1, &j.lib, j.kernel, &j.why)) j.lib = nullptr;
+        if (!compile_load(sum_product_source(*plan), plan->device, names, 1, &j.lib, &j.kernel, &j.why)) j.lib = nullptr;
     }
-    return j.lib ? j.kernel[0] : nullptr;
+    return j.lib ? j.kernel : nullptr;
 }
 
 int specialised_kernel_ready(const ck_ldpc_plan* plan, int place, const void** out) {
@@ -618,11 +619,14 @@ int specialised_kernel_ready(const ck_ldpc_plan* plan, int place, const void** o
     const int mode = effective_mode(plan->jit_mode);
     if (mode == CK_LDPC_SPECIALISE_OFF) return CK_OK;
     std::lock_guard<std::mutex> lock(plan->jit_mu);
-    const ck_ldpc_plan::Jit& j = plan->jit;
+    const ck_ldpc_plan::Jit& j = plan->jit[place];
     if (j.tried && j.lib) {
-        *out = j.kernel[place];
+        *out = j.kernel;
         return CK_OK;
     }
+    // Compiled for another placement only: the table-driven kernel.
+    if (!j.tried && std::any_of(std::begin(plan->jit), std::end(plan->jit), [](const auto& k) { return k.lib != nullptr; }))
+        return CK_OK;
     if (mode == CK_LDPC_SPECIALISE_ON)
         return ck::fail(CK_ERR_UNSUPPORTED,
                         j.tried ? "code-specialised decoder unavailable: %s"
@@ -690,14 +694,10 @@ void forget_plan_kernels(const ck_ldpc_plan* plan) {
         }
         it = g_mixed.erase(it);
     }
-    if (plan->jit.lib) {
-        for (const void* k : plan->jit.kernel)
-            if (k) ck::forget_kernel(k);
-        (void)cudaLibraryUnload(plan->jit.lib);
-    }
-    if (plan->jit_sp.lib) {
-        ck::forget_kernel(plan->jit_sp.kernel[0]);
-        (void)cudaLibraryUnload(plan->jit_sp.lib);
+    for (const ck_ldpc_plan::Jit* j : {&plan->jit[0], &plan->jit[1], &plan->jit[2], &plan->jit[3], &plan->jit_sp}) {
+        if (!j->lib) continue;
+        ck::forget_kernel(j->kernel);
+        (void)cudaLibraryUnload(j->lib);
     }
 }
 

@@ -501,8 +501,13 @@ extern "C" int ck_ldpc_plan_get_specialise(const ck_ldpc_plan* plan, int32_t* mo
     if (!plan || !mode || !state) return ck::fail(CK_ERR_INVALID_ARGUMENT, "NULL argument");
     std::lock_guard<std::mutex> lock(plan->jit_mu);
     *mode = plan->jit_mode;
-    *state = !plan->jit.tried ? 0 : (plan->jit.lib ? 1 : -1);
-    if (*state < 0) (void)ck::fail(CK_ERR_UNSUPPORTED, "%s", plan->jit.why.c_str());
+    *state = 0;
+    for (const ck_ldpc_plan::Jit& j : plan->jit) {
+        if (j.lib) *state = 1;
+        if (*state == 1 || !j.tried) continue;
+        *state = -1;
+        (void)ck::fail(CK_ERR_UNSUPPORTED, "%s", j.why.c_str());
+    }
     return CK_OK;
 }
 

@@ -362,7 +362,8 @@ int ck_ldpc_plan_resolved_launch(const ck_ldpc_plan* plan, int32_t rule, ck_ldpc
  * frame groups have one thread per row slot (threads per frame == Z rounded
  * up to whole warps) then run it, and sum-product decodes of small codes a
  * program of their own (compiled on the first of them; without it, in every
- * mode, the table-driven kernel serves).  AUTO (the default) falls back to the
+ * mode, the table-driven kernel serves).  Each message placement's kernel is
+ * compiled by the first decode that runs it.  AUTO (the default) falls back to the
  * table-driven kernel where NVRTC is missing or the environment sets
  * COMMKIT_GB300_SPECIALISE=0 (COMMKIT_GB300_NVRTC names the NVRTC library
  * to load instead of searching for it); ON makes an unavailable specialisation an

@@ -92,3 +92,27 @@ def test_no_workspace_for_messages_in_registers():
     for g in got:
         for name in ("bits", "llrs", "valid", "iterations"):
             np.testing.assert_array_equal(getattr(g, name).cpu().numpy(), getattr(want, name).cpu().numpy(), err_msg=name)
+
+
+@pytest.mark.parametrize("rule", ["sum_product", "min_sum"])
+def test_first_decode_inside_a_capture(rule):
+    """The first decode of a plan, which compiles its kernel, recorded in a
+    graph: the replay gives what a decode outside gives."""
+    import torch
+
+    import commkit_gb300 as ck
+
+    base = W.dual_diagonal_base(5, 13, 24, (3,) * 8, seed=11)
+    code = ck.LDPCCode.quasi_cyclic(base, lifting=24)
+    code._plan(0)  # plans allocate their tables outside captures
+    method = (ck.SumProduct if rule == "sum_product" else ck.MinSum)(max_iterations=8)
+    x = torch.from_numpy((1.2 + 1.5 * np.random.default_rng(9).standard_normal((40, code.n))).astype(np.float32)).cuda()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        r = ck.decode(x, code=code, method=method)
+    graph.replay()
+    torch.cuda.synchronize()
+    want = ck.decode(x, code=code, method=method)
+    for name in ("bits", "llrs", "valid", "iterations"):
+        np.testing.assert_array_equal(getattr(r, name).cpu().numpy(), getattr(want, name).cpu().numpy(), err_msg=name)
