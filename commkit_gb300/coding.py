@@ -456,9 +456,12 @@ class _Plan:
         return cfg.threads_per_frame, cfg.frames_per_block, cfg.placement
 
     def resolved_launch(self, rule: int = _lib.CK_LDPC_MIN_SUM) -> tuple[int, int, int]:
-        """(threads per frame, frames per block, placement) a decode by
-        ``rule`` runs with now: the setting resolved on the plan's device
-        (current), the placement the one actually used."""
+        """(threads per frame, frames per block, placement) a decode of a
+        large batch by ``rule`` runs with now: the setting resolved on the
+        plan's device (current), the placement the one used.  Setting the
+        three selects the same kernel.  With no threads set, short min-sum
+        batches and sum-product decodes of small circulant codes keep their
+        messages in registers instead (one frame per block)."""
         cfg = _lib.Launch()
         st = _lib.lib().ck_ldpc_plan_resolved_launch(self.handle, int(rule), ctypes.byref(cfg))
         _lib.check(st, "resolved_launch")

@@ -177,6 +177,7 @@ int device_limits(int dev, int* sms, int* smem_optin) {
 // frames by `rule`; a pure function of the plan, its launch setting, the
 // rule and B.  may_compile false: a code-specialised kernel only if one is
 // compiled already (no NVRTC, no module load), and nothing cached.
+// registers false: as if the code had no register form.
 int resolve_shape(const ck_ldpc_plan* plan, int32_t rule, Resolved* r, int* per_sm_out, int* sms_out,
                   bool may_compile);
 
@@ -189,7 +190,8 @@ int32_t ell_threads(const ck_ldpc_plan* plan, int32_t frames) {
     return std::max(32, std::min(most / std::max(1, frames) / 32 * 32, rows));
 }
 
-int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool may_compile = true) {
+int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool may_compile = true,
+            bool registers = true) {
     if (rule != CK_LDPC_MIN_SUM && rule != CK_LDPC_SUM_PRODUCT)
         return ck::fail(CK_ERR_INVALID_ARGUMENT, "unknown check rule %d", rule);
     static_assert(sizeof(Resolved) <= sizeof(plan->shape_cache[0].resolved), "shape cache too small");
@@ -247,7 +249,7 @@ int resolve(const ck_ldpc_plan* plan, int32_t rule, int64_t B, Resolved* r, bool
     // The register form (one frame per block): sum-product batches of every
     // size, min-sum batches of up to reg_waves, where the time of a frame
     // counts for more than the frames an SM holds.
-    const bool regs = r->reg_kernel && B > 0 &&
+    const bool regs = registers && r->reg_kernel && B > 0 &&
                       (rule == CK_LDPC_SUM_PRODUCT || B <= int64_t(sms) * r->reg_per_sm * reg_waves(plan, r->reg_T));
     r->direct = regs && B <= int64_t(sms) * r->reg_per_sm;
     if (regs) {
@@ -1082,7 +1084,9 @@ extern "C" int ck_ldpc_plan_resolved_launch(const ck_ldpc_plan* plan, int32_t ru
         return ck::fail(CK_ERR_INVALID_ARGUMENT, "plan is for device %d, current device is %d", plan->device,
                         device);
     Resolved r;
-    CK_TRY(resolve(plan, rule, int64_t(1) << 40, &r));  // a full batch: the shape before any spreading of a short one
+    // A full batch without the register form: the shape before any spreading
+    // of a short one, which the same three values set.
+    CK_TRY(resolve(plan, rule, int64_t(1) << 40, &r, true, false));
     out->threads_per_frame = r.T;
     out->frames_per_block = r.G;
     out->placement = !r.r_smem ? CK_LDPC_PLACE_GLOBAL : (r.edges ? CK_LDPC_PLACE_EDGES : CK_LDPC_PLACE_SHARED);

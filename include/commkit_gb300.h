@@ -346,10 +346,15 @@ typedef struct ck_ldpc_launch {
 int ck_ldpc_plan_set_launch(ck_ldpc_plan* plan, const ck_ldpc_launch* launch);
 int ck_ldpc_plan_get_launch(const ck_ldpc_plan* plan, ck_ldpc_launch* launch);
 /*
- * The shape a plain decode by `rule` (CK_LDPC_MIN_SUM / CK_LDPC_SUM_PRODUCT)
- * runs with under the current setting, resolved (and its code-specialised
- * kernel compiled, when it has one): threads per frame, frames per block
- * and the placement actually used (SHARED, GLOBAL or EDGES, never AUTO).
+ * The shape a plain decode of a large batch by `rule` (CK_LDPC_MIN_SUM /
+ * CK_LDPC_SUM_PRODUCT) runs with under the current setting, resolved (and its
+ * code-specialised kernel compiled, when it has one): threads per frame,
+ * frames per block and the placement used (SHARED, GLOBAL or EDGES, never
+ * AUTO); setting these values selects the same kernel.  Short batches run
+ * fewer frames per block.  With no threads set, min-sum decodes of short
+ * batches and sum-product decodes of small circulant codes keep their
+ * messages in registers instead, one frame per block and two lanes per row
+ * (the shape reported is then the table-driven sum-product kernel's).
  * The plan's device must be current.  No reference counterpart.
  */
 int ck_ldpc_plan_resolved_launch(const ck_ldpc_plan* plan, int32_t rule, ck_ldpc_launch* launch);

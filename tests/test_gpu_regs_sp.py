@@ -116,3 +116,23 @@ def test_first_decode_inside_a_capture(rule):
     want = ck.decode(x, code=code, method=method)
     for name in ("bits", "llrs", "valid", "iterations"):
         np.testing.assert_array_equal(getattr(r, name).cpu().numpy(), getattr(want, name).cpu().numpy(), err_msg=name)
+
+
+@pytest.mark.parametrize("rule", [0, 1])
+def test_resolved_launch_can_be_set(rule):
+    """The reported shape is one kernel's, which setting it selects."""
+    import torch
+
+    import commkit_gb300 as ck
+
+    code = ck.LDPCCode.quasi_cyclic(W.dual_diagonal_base(5, 13, 72, (3,) * 8, seed=13), lifting=72)
+    plan = code._plan(0)
+    method = ck.MinSum(max_iterations=5) if rule == 0 else ck.SumProduct(max_iterations=5)
+    x = torch.from_numpy((1.2 + 1.5 * np.random.default_rng(9).standard_normal((70, code.n))).astype(np.float32)).cuda()
+    want = ck.decode(x, code=code, method=method)
+    shape = plan.resolved_launch(rule)
+    plan.set_launch(*shape)
+    assert plan.resolved_launch(rule) == shape
+    got = ck.decode(x, code=code, method=method)
+    for name in ("bits", "llrs", "valid", "iterations"):
+        np.testing.assert_array_equal(getattr(got, name).cpu().numpy(), getattr(want, name).cpu().numpy(), err_msg=name)
