@@ -2,7 +2,9 @@
 
 Every launch shape gives bit-identical results, so picking one is purely a
 speed question.  :func:`tune` times the candidates for one code on the
-current GPU: threads per frame (divisors and multiples of the lifting
+current GPU: the shape the plan picks by itself, which also lets short
+batches and sum-product decodes keep their messages in registers, and set
+ones: threads per frame (divisors and multiples of the lifting
 rounded up to whole warps), frames per block, and where the check-message
 state lives.  It stores the fastest in a JSON cache keyed by the GPU's name
 and a digest of the code's schedule.  :func:`apply_cached` (called when a
@@ -173,7 +175,7 @@ def tune(code: Any, *, device: int = 0, frames: int | None = None, iterations: i
     method = MinSum(max_iterations=iterations, early_stop=True)
     ws = None
     results = []
-    for t, g, place in candidates(info):
+    for t, g, place in [(0, 0, _lib.CK_LDPC_PLACE_AUTO), *candidates(info)]:
         try:
             plan.set_launch(t, g, place)
             need = plan.workspace_size(frames)
@@ -195,7 +197,10 @@ def tune(code: Any, *, device: int = 0, frames: int | None = None, iterations: i
     if not results:
         plan.set_launch(0, 0, 0)
         raise RuntimeError("tune(): no launch shape fits this code")
-    ms, t, g, place, its = min(results)
+    # A set shape holds for every batch and rule, the plan's own follows them:
+    # it stays unless a set one is 5 % faster (what timings of short batches,
+    # which the host's calls bound, repeat to).
+    ms, t, g, place, its = min(results, key=lambda r: r[0] * (1.0 if r[1:4] == (0, 0, 0) else 1.05))
     best = {
         "threads_per_frame": t, "frames_per_block": g, "placement": place, "ms": ms,
         "edge_updates_per_s": its * info["num_edges"] / (ms * 1e-3),

@@ -74,3 +74,19 @@ def test_tuning_batch_sits_in_the_waterfall():
     its = res.iterations.cpu().numpy()
     assert 0.2 < fer < 0.8, fer
     assert its.min() < 25 and its.max() == 50
+
+
+@pytest.mark.gpu
+def test_tune_times_the_plans_own_shape(tmp_path, monkeypatch):
+    """A code of short lifting, whose batches the plan's own shape decodes
+    with their messages in registers at two thirds of the time of the forms
+    that can be set: the own shape stays, also for a fresh code object."""
+    import commkit_gb300 as ck
+
+    monkeypatch.setenv("COMMKIT_GB300_TUNING", str(tmp_path / "t.json"))
+    base = W.dual_diagonal_base(16, 32, 16, (3,) * 16, seed=16)
+    code = ck.LDPCCode.quasi_cyclic(base, lifting=16)
+    best = tuning.tune(code, device=0, frames=9728, iterations=20, reps=5)
+    assert (best["threads_per_frame"], best["frames_per_block"], best["placement"]) == (0, 0, 0)
+    assert code._plan(0).get_launch() == (0, 0, 0)
+    assert ck.LDPCCode.quasi_cyclic(base, lifting=16)._plan(0).get_launch() == (0, 0, 0)
