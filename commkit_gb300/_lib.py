@@ -53,6 +53,7 @@ EXPORTS = (
     "ck_llr_separable_frames",
     "ck_llr_points",
     "ck_llr_points_frames",
+    "ck_llr_points_priors",
     "ck_random_bits",
     "ck_ldpc_encode",
     "ck_ldpc_encode_checked",
@@ -202,6 +203,7 @@ def _declare(lib: ctypes.CDLL) -> None:
             ctypes.c_int),
         "ck_llr_points": ([p, i64, p, p, p, i32, i32, ctypes.c_float, i32, p, p], ctypes.c_int),
         "ck_llr_points_frames": ([p, i64, i64, p, p, p, p, i32, i32, i32, p, p], ctypes.c_int),
+        "ck_llr_points_priors": ([p, i64, i64, p, f32, p, p, p, i32, i32, p, p], ctypes.c_int),
         "ck_random_bits": ([p, i64, ctypes.c_uint64, ctypes.c_uint64, p], ctypes.c_int),
         "ck_ldpc_encode": ([p, i64, i32, i32, i32, p, p, i32, p, p, ctypes.c_size_t, p, p], ctypes.c_int),
         "ck_ldpc_encode_checked": ([p, i64, i32, i32, i32, p, p, i32, p, p, p], ctypes.c_int),
@@ -308,7 +310,7 @@ def _load_calls(handle: ctypes.CDLL):
 
     mod.init(addr(handle.ck_ldpc_decode), addr(handle.ck_ldpc_workspace_size),
              addr(handle.ck_llr_separable_maxlog), addr(handle.ck_llr_separable), addr(handle.ck_llr_points),
-             DecodeResult)  # fmt: skip
+             addr(handle.ck_llr_points_priors), DecodeResult)  # fmt: skip
     return mod
 
 

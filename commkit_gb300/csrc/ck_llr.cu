@@ -58,7 +58,7 @@ CK_LLR_EXTERN(6)
 namespace points {
 #define CK_LLR_POINTS_EXTERN(K)                                                               \
     extern template int launch_points<K>(const float2*, uint32_t, const Table&, const NoiseScale&, \
-                                         bool, float*, cudaStream_t);
+                                         Form, float*, cudaStream_t);
 CK_LLR_POINTS_EXTERN(1) CK_LLR_POINTS_EXTERN(2) CK_LLR_POINTS_EXTERN(3) CK_LLR_POINTS_EXTERN(4)
 CK_LLR_POINTS_EXTERN(5) CK_LLR_POINTS_EXTERN(6) CK_LLR_POINTS_EXTERN(7) CK_LLR_POINTS_EXTERN(8)
 CK_LLR_POINTS_EXTERN(9) CK_LLR_POINTS_EXTERN(10) CK_LLR_POINTS_EXTERN(11) CK_LLR_POINTS_EXTERN(12)
@@ -128,7 +128,7 @@ int frame_noise(int64_t n, int64_t frame_len, const float* inv_s2, NoiseScale* s
 }
 
 int launch_points(const void* x, int64_t n, const void* pts, const float* log_pmf,
-                  const int32_t* labels, int32_t M, int32_t k, int32_t exact, const NoiseScale& noise,
+                  const int32_t* labels, int32_t M, int32_t k, points::Form form, const NoiseScale& noise,
                   float* out, void* stream) {
     if (k < 1 || k > CK_LLR_MAX_K)
         return ck::fail(CK_ERR_INVALID_ARGUMENT, "bits per symbol must be in [1, %d], got %d",
@@ -147,10 +147,9 @@ int launch_points(const void* x, int64_t n, const void* pts, const float* log_pm
     const float2* xs = static_cast<const float2*>(x);
     const uint32_t nn = static_cast<uint32_t>(n);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool ex = exact != 0;
     switch (k) {
 #define CK_CASE(K) \
-    case K: return points::launch_points<K>(xs, nn, t, noise, ex, out, s);
+    case K: return points::launch_points<K>(xs, nn, t, noise, form, out, s);
         CK_CASE(1) CK_CASE(2) CK_CASE(3) CK_CASE(4) CK_CASE(5) CK_CASE(6) CK_CASE(7) CK_CASE(8)
         CK_CASE(9) CK_CASE(10) CK_CASE(11) CK_CASE(12) CK_CASE(13) CK_CASE(14) CK_CASE(15) CK_CASE(16)
 #undef CK_CASE
@@ -174,6 +173,7 @@ using ck::llr::frame_noise;
 using ck::llr::check_lo_hi;
 using ck::llr::launch_points;
 using ck::llr::NoiseScale;
+using ck::llr::points::Form;
 
 extern "C" int ck_llr_separable_maxlog(const void* x, int64_t n, const ck_axis_maxlog* re,
                                        const ck_axis_maxlog* im, float inv_s2, float* out,
@@ -219,8 +219,8 @@ extern "C" int ck_llr_points(const void* x, int64_t n, const void* points, const
                              const int32_t* labels, int32_t M, int32_t k, float inv_s2,
                              int32_t exact, float* out, void* stream) {
     ck::clear_error();
-    return launch_points(x, n, points, log_pmf, labels, M, k, exact, scalar_noise(inv_s2), out,
-                         stream);
+    return launch_points(x, n, points, log_pmf, labels, M, k, exact ? Form::kExact : Form::kMaxLog,
+                         scalar_noise(inv_s2), out, stream);
 }
 
 extern "C" int ck_llr_points_frames(const void* x, int64_t n, int64_t frame_len,
@@ -230,5 +230,14 @@ extern "C" int ck_llr_points_frames(const void* x, int64_t n, int64_t frame_len,
     ck::clear_error();
     NoiseScale s;
     CK_TRY(frame_noise(n, frame_len, inv_s2, &s));
-    return launch_points(x, n, points, log_pmf, labels, M, k, exact, s, out, stream);
+    return launch_points(x, n, points, log_pmf, labels, M, k, exact ? Form::kExact : Form::kMaxLog, s, out, stream);
+}
+
+extern "C" int ck_llr_points_priors(const void* x, int64_t n, int64_t frame_len, const float* frame_inv_s2,
+                                    float inv_s2, const void* points, const float* log_pmf,
+                                    const int32_t* labels, int32_t M, int32_t k, float* out, void* stream) {
+    ck::clear_error();
+    NoiseScale s = scalar_noise(inv_s2);
+    if (frame_inv_s2) CK_TRY(frame_noise(n, frame_len, frame_inv_s2, &s));
+    return launch_points(x, n, points, log_pmf, labels, M, k, Form::kMaxLogPriors, s, out, stream);
 }

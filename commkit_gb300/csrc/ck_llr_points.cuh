@@ -464,13 +464,17 @@ __device__ __forceinline__ void store_row(float* row, const float* o, bool vec) 
 // order) two adjacent symbols per step (exact_sorted2); otherwise one
 // symbol in point order.  `vec`: rows of K floats may be stored as float4 /
 // float2 (out 16-byte aligned).
-template <int K, bool EXACT, bool SMEM>
+// EQUAL: with the form for one prior.  Its registers leave the form for priors
+// half to three quarters of its blocks (128 points: 86 against 56), which costs
+// that one 3 to 7 % (2^22 symbols, 32 / 128 / 512 points 57 / 196 / 706 against
+// 55 / 184 / 686 us), so callers that know their priors differ leave it out.
+template <int K, bool EXACT, bool SMEM, bool EQUAL = true>
 __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __restrict__ x, uint32_t n,
                                                               const Table t, const NoiseScale noise,
                                                               float* __restrict__ out, bool vec) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int L = 1 << K;
-    using C = Cross<K>;
+    using C = Cross<EQUAL && !EXACT ? K : 1>;
     __shared__ int s_bad, s_ident, s_same, s_cross;
     __shared__ __align__(16) float2 s_lev[2][(C::N + 1) / 2 * 2];  // the cross's coordinates, each twice
     __shared__ __align__(8) float s_nz[2];
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __re
                 }
                 const float2 p = t.pts[m];
                 const float l = t.logp[m];
-                if (!EXACT && l != t.logp[0]) s_same = 0;
+                if (EQUAL && !EXACT && l != t.logp[0]) s_same = 0;
                 if (EXACT) {
                     ri[lab] = make_float4(p.x, p.x, p.y, p.y);
                     lp[lab] = make_float2(l, l);
@@ -536,7 +540,7 @@ __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __re
                 return;
             }
         } else {
-            if (s_bad == 0 && s_same) {
+            if (EQUAL && s_bad == 0 && s_same) {
                 // One prior for all points: two symbols per step by distance.
                 const float lp0 = t.logp[0];
                 for (int m = threadIdx.x; m < L; m += blockDim.x) {
@@ -657,9 +661,12 @@ __global__ void __launch_bounds__(kThreads) llr_points_kernel(const float2* __re
     }
 }
 
+// The LLRs wanted: max-log, exact, or max-log of points whose priors differ.
+enum class Form { kMaxLog, kExact, kMaxLogPriors };
+
 // Launch for K bits per symbol (defined in ck_llr_points_lo.cu / _hi.cu).
 template <int K>
-int launch_points(const float2* x, uint32_t n, const Table& t, const NoiseScale& noise, bool exact,
+int launch_points(const float2* x, uint32_t n, const Table& t, const NoiseScale& noise, Form form,
                   float* out, cudaStream_t stream);
 
 }  // namespace points

@@ -45,6 +45,7 @@ decltype(&ck_ldpc_workspace_size) g_workspace_size = nullptr;
 decltype(&ck_llr_separable_maxlog) g_llr_maxlog = nullptr;
 decltype(&ck_llr_separable) g_llr_levels = nullptr;
 decltype(&ck_llr_points) g_llr_points = nullptr;
+decltype(&ck_llr_points_priors) g_llr_priors = nullptr;
 PyTypeObject* g_result_type = nullptr;  // DecodeResult
 PyObject* g_empty = nullptr;            // ()
 PyObject* g_names[5] = {};              // bits, llrs, valid, iterations, checked
@@ -94,11 +95,11 @@ PyObject* bad_call(const char* what) {
     return nullptr;
 }
 
-// init(decode, workspace_size, llr_separable_maxlog, llr_separable, llr_points, DecodeResult)
+// init(decode, workspace_size, llr_separable_maxlog, llr_separable, llr_points, llr_points_priors, DecodeResult)
 PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t na) {
-    if (na != 6 || !PyType_Check(a[5])) return bad_call("init(5 entry-point addresses, DecodeResult)");
-    void* p[5];
-    for (int i = 0; i < 5; ++i) {
+    if (na != 7 || !PyType_Check(a[6])) return bad_call("init(6 entry-point addresses, DecodeResult)");
+    void* p[6];
+    for (int i = 0; i < 6; ++i) {
         p[i] = PyLong_AsVoidPtr(a[i]);
         if (PyErr_Occurred()) return nullptr;
         if (!p[i]) return bad_call("init(): NULL entry point");
@@ -108,8 +109,9 @@ PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t na) {
     g_llr_maxlog = reinterpret_cast<decltype(g_llr_maxlog)>(p[2]);
     g_llr_levels = reinterpret_cast<decltype(g_llr_levels)>(p[3]);
     g_llr_points = reinterpret_cast<decltype(g_llr_points)>(p[4]);
-    Py_INCREF(a[5]);
-    Py_XSETREF(g_result_type, reinterpret_cast<PyTypeObject*>(a[5]));
+    g_llr_priors = reinterpret_cast<decltype(g_llr_priors)>(p[5]);
+    Py_INCREF(a[6]);
+    Py_XSETREF(g_result_type, reinterpret_cast<PyTypeObject*>(a[6]));
     Py_RETURN_NONE;
 }
 
@@ -222,7 +224,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t na) {
 //   entries: list indexed by device of (kind, exact, p0, p1, p2, M, k) or
 //   None; kind 0 closed-form max-log (p0/p1 the axis structs), 1 per-axis
 //   levels (p0/p1 the axis structs), 2 every point (p0 points, p1 log_pmf,
-//   p2 labels).
+//   p2 labels), 3 the same, max-log of points whose priors differ.
 PyObject* llr(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (na != 3 || !PyList_Check(a[2])) return bad_call("llr(symbols, noise_var, entries: list)");
     if (!g_llr_maxlog) return bad_call("llr(): init() was not called");
@@ -289,6 +291,10 @@ PyObject* llr(PyObject*, PyObject* const* a, Py_ssize_t na) {
             st = g_llr_points(x, n, ptr(2), static_cast<const float*>(ptr(3)), static_cast<const int32_t*>(ptr(4)),
                               static_cast<int32_t>(M), static_cast<int32_t>(k), inv_s2, static_cast<int32_t>(exact),
                               o, s);
+        else if (kind == 3)
+            st = g_llr_priors(x, n, 0, nullptr, inv_s2, ptr(2), static_cast<const float*>(ptr(3)),
+                              static_cast<const int32_t*>(ptr(4)), static_cast<int32_t>(M), static_cast<int32_t>(k), o,
+                              s);
         else
             Py_RETURN_NONE;
     }

@@ -636,6 +636,30 @@ def _llr_separable_gpu(symbols: Any, x: _device.DeviceArray, c: Constellation, n
     return out
 
 
+def _priors_differ(c: Constellation) -> bool:
+    """Whether the points' float32 log priors are not all the same."""
+    d = c.__dict__.get("_priors_differ")
+    if d is None:
+        logp = host_tables(c, "points")[1]
+        d = c.__dict__["_priors_differ"] = bool((logp != logp[0]).any())
+    return d
+
+
+def points_llr(c: Constellation, method: str, x: int, n: int, tables: tuple, out: int, stream: int, *,
+               inv_s2: float = 0.0, frame_len: int = 0, frames: int | None = None) -> int:  # fmt: skip
+    """The M-point demapper's C call on device addresses: one ``inv_s2``, or
+    one per frame of ``frame_len`` symbols at ``frames``; returns the status."""
+    lib = _lib.lib()
+    p = [t.data_ptr() for t in tables]
+    k = c.bits_per_symbol
+    if method == "maxlog" and _priors_differ(c):
+        return lib.ck_llr_points_priors(x, n, frame_len, frames, inv_s2, *p, c.order, k, out, stream)
+    exact = 1 if method == "exact" else 0
+    if frames is None:
+        return lib.ck_llr_points(x, n, *p, c.order, k, inv_s2, exact, out, stream)
+    return lib.ck_llr_points_frames(x, n, frame_len, frames, *p, c.order, k, exact, out, stream)
+
+
 def _llr_points_gpu(symbols: Any, x: _device.DeviceArray, c: Constellation, nv: float,
                     method: str) -> Any:  # fmt: skip
     """``commkit/mapping/_demap.py:150-219`` (the GPU branch) on the
@@ -654,12 +678,11 @@ def _llr_points_gpu(symbols: Any, x: _device.DeviceArray, c: Constellation, nv: 
     od = _device.wrap(out, "out")
     with _device.on_device(x):
         pts, logp, lab = device_tables(c, "points", x)
-        st = _lib.lib().ck_llr_points(fx.ptr, n, pts.data_ptr(), logp.data_ptr(), lab.data_ptr(),
-                                      c.order, k, inv_s2(nv), 1 if method == "exact" else 0, od.ptr,
-                                      _device.stream_of(x))  # fmt: skip
+        st = points_llr(c, method, fx.ptr, n, (pts, logp, lab), od.ptr, _device.stream_of(x), inv_s2=inv_s2(nv))
         _lib.check(st, "compute_llr()")
     if x.kind == "torch" and x.contiguous and x.dtype == np.complex64:
-        _register_calls(c, method, x.device, (2, 1 if method == "exact" else 0, pts.data_ptr(), logp.data_ptr(),
+        kind = 3 if method == "maxlog" and _priors_differ(c) else 2
+        _register_calls(c, method, x.device, (kind, 1 if method == "exact" else 0, pts.data_ptr(), logp.data_ptr(),
                                               lab.data_ptr(), c.order, k))  # fmt: skip
     shape = tuple(x.shape[:-1]) + (x.shape[-1] * k,) if x.ndim else (k,)
     return out.reshape(shape)
@@ -733,10 +756,7 @@ def compute_llr_frames(symbols: Any, *, noise_var: Any = None, constellation: Co
         stream = _device.stream_of(x)
         lib = _lib.lib()
         if kind == "points":
-            pts, logp, lab = tables
-            st = lib.ck_llr_points_frames(x.ptr, F * S, S, sd.ptr, pts.data_ptr(), logp.data_ptr(),
-                                          lab.data_ptr(), constellation.order, k,
-                                          1 if method == "exact" else 0, od.ptr, stream)  # fmt: skip
+            st = points_llr(constellation, method, x.ptr, F * S, tables, od.ptr, stream, frame_len=S, frames=sd.ptr)
             _lib.check(st, "compute_llr_frames()")
             return out
         half = len(tables) // 2

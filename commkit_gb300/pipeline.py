@@ -39,7 +39,8 @@ import numpy as np
 
 from . import _device, _lib
 from .coding import DecodeResult, LDPCCode, MinSum, _require_leading_info, _rule_args, decode_mixed
-from .mapping import Constellation, _axis_struct, _table_kind, compute_llr_frames, device_tables, inv_s2_frames
+from .mapping import (Constellation, _axis_struct, _table_kind, compute_llr_frames, device_tables, inv_s2_frames,
+                      points_llr)  # fmt: skip
 
 
 @dataclass
@@ -180,9 +181,7 @@ class MixedReceiver:
                 exact = 1 if s.demap == "exact" else 0
                 x, s2, out = self.sym[i].data_ptr(), self.s2[i].data_ptr(), self.llr[i].data_ptr()
                 if kind == "points":
-                    st_ = lib.ck_llr_points_frames(x, F * S, S, s2, tabs[0].data_ptr(), tabs[1].data_ptr(),
-                                                   tabs[2].data_ptr(), s.constellation.order,
-                                                   s.constellation.bits_per_symbol, exact, out, st)  # fmt: skip
+                    st_ = points_llr(s.constellation, s.demap, x, F * S, tabs, out, st, frame_len=S, frames=s2)
                 else:
                     half = len(tabs) // 2
                     re, im = _axis_struct(tabs[:half], kind), _axis_struct(tabs[half:], kind)

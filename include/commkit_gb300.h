@@ -143,6 +143,12 @@ int ck_llr_points(const void* x, int64_t n, const void* points, const float* log
 int ck_llr_points_frames(const void* x, int64_t n, int64_t frame_len, const float* inv_s2,
                          const void* points, const float* log_pmf, const int32_t* labels,
                          int32_t M, int32_t k, int32_t exact, float* out, void* stream);
+/* Max-log as ck_llr_points (frame_inv_s2 NULL) or ck_llr_points_frames, for a
+ * caller that knows its priors differ: the same results from a kernel without
+ * the form for equal priors. */
+int ck_llr_points_priors(const void* x, int64_t n, int64_t frame_len, const float* frame_inv_s2, float inv_s2,
+                         const void* points, const float* log_pmf, const int32_t* labels, int32_t M,
+                         int32_t k, float* out, void* stream);
 
 /* ---------------------------------------------------------------------- */
 /* Coded-link simulation (the Monte-Carlo error-rate loop)                 */

@@ -152,3 +152,47 @@ def test_frames_match_single_calls(torch_dev):
             np.testing.assert_allclose(both.reshape(F * S, -1)[:S], oracle_llr(c, x[0], float(nv[0]), method),
                                        **TOL)  # fmt: skip
     assert inv_s2(0.0) == np.float32(1e20)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 5, 7, 9, 12])
+@pytest.mark.parametrize("n", [1, 255, 20001])
+def test_kernel_without_the_equal_prior_form(k, n, monkeypatch):
+    """ck_llr_points_priors gives ck_llr_points' max-log LLRs bit for bit,
+    one noise value or one per frame, and is what points of differing priors
+    run; equal priors keep ck_llr_points."""
+    import torch
+
+    import commkit_gb300 as ck
+    from commkit_gb300 import _device, _lib
+
+    M = 1 << k
+    rng = np.random.default_rng(k)
+    pts = (rng.standard_normal(M) + 1j * rng.standard_normal(M)).astype(np.complex64)
+    lab = ((rng.permutation(M)[:, None] >> np.arange(k)[::-1]) & 1).astype(np.int8)
+    x = torch.from_numpy((rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64)).cuda()
+    lib, stream = _lib.lib(), _device.stream_of(_device.wrap(x))
+    frame = torch.from_numpy(rng.uniform(1.0, 9.0, n).astype(np.float32)).cuda()
+    d = [torch.from_numpy(a).cuda() for a in (pts, np.log(rng.dirichlet(np.ones(M))).astype(np.float32),
+                                              (lab @ (1 << np.arange(k)[::-1])).astype(np.int32))]  # fmt: skip
+    p = [a.data_ptr() for a in d]
+    out = torch.zeros((4, n, k), dtype=torch.float32, device="cuda")
+    o = [out[i].data_ptr() for i in range(4)]
+    _lib.check(lib.ck_llr_points(x.data_ptr(), n, *p, M, k, 3.0, 0, o[0], stream), "points")
+    _lib.check(lib.ck_llr_points_priors(x.data_ptr(), n, 0, None, 3.0, *p, M, k, o[1], stream), "priors")
+    _lib.check(lib.ck_llr_points_frames(x.data_ptr(), n, 1, frame.data_ptr(), *p, M, k, 0, o[2], stream), "frames")
+    _lib.check(lib.ck_llr_points_priors(x.data_ptr(), n, 1, frame.data_ptr(), 0.0, *p, M, k, o[3], stream), "priors")
+    bits = out.cpu().numpy().view(np.uint32)
+    np.testing.assert_array_equal(bits[1], bits[0])
+    np.testing.assert_array_equal(bits[3], bits[2])
+
+    monkeypatch.setenv("COMMKIT_GB300_CALLS", "0")
+    calls = []
+    for name in ("ck_llr_points", "ck_llr_points_priors"):
+        f = getattr(lib, name)
+        monkeypatch.setattr(lib, name, lambda *a, f=f, name=name: (calls.append(name), f(*a))[1])
+    pmf = rng.dirichlet(np.ones(M))
+    for c in (ck.Constellation(pts, lab, pmf), ck.Constellation(pts, lab)):
+        if c._axes is None:
+            ck.compute_llr(x, noise_var=0.3, constellation=c, method="maxlog")
+            differ = c.pmf is not None and np.ptp(np.asarray(c.pmf)) > 0
+            assert calls.pop() == ("ck_llr_points_priors" if differ else "ck_llr_points")
