@@ -92,3 +92,27 @@ def test_staircase_codes_equal_oracle(N, m, weight, punctured, frames, placement
                    r.iterations.cpu().numpy().reshape(-1))  # fmt: skip
             for g, w, what in zip(got, want, ("bits", "llrs", "valid", "iterations"), strict=True):
                 np.testing.assert_array_equal(g.reshape(w.shape), w, err_msg=f"{what}, {threads} threads")
+
+
+@pytest.mark.parametrize("N,m,weight", [(6000, 3000, 3), (3000, 750, 4), (64800, 32400, 3)])
+def test_not_a_number_counts_as_absent(N, m, weight):
+    """NaN and infinite LLRs, which meet in rows: a NaN magnitude changes no
+    minimum, as in the oracle."""
+    import torch
+
+    import commkit_gb300 as ck
+
+    code = staircase_code(ck, N, m, weight, seed=N)
+    rng = np.random.default_rng(11)
+    llrs = (2.0 + 2.0 * rng.standard_normal((3, code.n))).astype(np.float32)
+    llrs[0, rng.integers(0, N, 40)] = np.nan
+    llrs[1, rng.integers(0, N, 40)] = np.inf
+    llrs[1, rng.integers(0, N, 40)] = -np.inf
+    llrs[2, N - 3 :] = [np.nan, np.inf, -np.inf]
+    row_ptr, cols, _ = code._schedule
+    method = ck.MinSum(max_iterations=5)
+    r = ck.decode(torch.from_numpy(llrs).cuda(), code=code, method=method)
+    want = oracle.decode(llrs, (row_ptr, cols, N), k=code.k, scale=method.scale, offset=method.offset, max_iterations=5,
+                         early_stop=True)  # fmt: skip
+    for g, w in zip((r.bits, r.llrs, r.valid, r.iterations), want, strict=True):
+        np.testing.assert_array_equal(g.cpu().numpy().reshape(w.shape), w)
