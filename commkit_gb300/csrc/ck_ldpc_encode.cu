@@ -16,7 +16,8 @@
 // accumulators (lifted codes, g = Z) split over blocks, each packing the
 // group's information anew (from L2).  The rows of a tile go in chunks of
 // four rows per thread, whose column loads are in flight together, each chunk
-// scanned over its chains in shared memory.  Measured (encode_blocks): 1000 frames
+// scanned over its chains in shared memory.  Measured (encode_blocks, calls
+// back to back; the figures above are of each kernel alone, cold): 1000 frames
 // of code C 130 to 31 us, 4096 frames of code A 31 to 14 us (the launch), 128
 // frames of DVB-S2 normal 97 to 64 us.  A few frames of one long chain
 // keep the byte-wise kernels (few_long_frames, ck_sim.cu).

@@ -106,7 +106,8 @@ constexpr int kPlaceEdges = 2;  // one message per edge in shared memory
 constexpr int kPlaceRegisters = 3;  // one message per edge in registers (decode_regs_body)
 // Threads per frame of a circulant plan's register form (two lanes per row,
 // whole warps of 16 rows), or 0 where it has none: more than kRegSlots edges
-// per lane, or a longest row above kPackedDegree.
+// per lane, or a longest row above kPackedDegree.  (Up to there it gains, also
+// where its threads leave fewer registers than slots: ck_ldpc_regs.cuh.)
 constexpr int kRegSlots = 72;
 int32_t register_threads(const ck_ldpc_plan& plan);
 // The plan's code-specialised min-sum kernel for a row-degree bound and a

@@ -87,8 +87,12 @@ __device__ __forceinline__ void reg_edge(const RegOut& o, const float q, const u
 // row a frame's iteration is the chain of a row's calls, layer after layer;
 // here it is half of that, all base rows of a layer run theirs together, and
 // degrees are constants (the table-driven kernel steps through its degree
-// bound).  Every size gains, so there is no limit of waves.  50 iterations,
-// table-driven kernel against this one: code B (Z = 96) at 3.2 dB 1 frame 75
+// bound).  Every size gains, so there is no limit of waves, and every code
+// measured: 8 iterations of 1 / 608 / 6000 frames, Z = 8 (69 slots) 366 / 370 /
+// 1050 to 90 / 91 / 483 us, Z = 256 (43 slots) 296 / 638 / 6223 to 82 / 314 / 3055,
+// also where the slots exceed the registers and spill, Z = 256 (65 slots) 447 /
+// 986 us to 149 / 540 for 1 / 608 frames, Z = 240 (72 slots) 496 / 1046 to 163 /
+// 605.  50 iterations, table-driven kernel against this one: code B (Z = 96) at 3.2 dB 1 frame 75
 // to 20 us, 256 frames 1159 to 255, 2048 1266 to 423, at 2.4 dB 2048 frames
 // 2417 to 1474; code A at 1.6 dB 16 frames 733 to 103 us, 1024 1581 to 478,
 // 4096 2289 to 1187.
