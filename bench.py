@@ -1220,6 +1220,59 @@ def measure_feed(codes, pool, sat_rate: float, duration: float, info_bits, dev, 
             "p99_ms_at_70pct": sweep["70%"]["p99_ms"], "launches": launches, "clocks": clk.summary()}  # fmt: skip
 
 
+def short_line(line: dict) -> dict:
+    """The result line with its figures and without the details (which go to
+    stderr whole): under 3,000 characters, so that the end of a log that keeps
+    a few thousand holds all of it."""
+
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.5g}")
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items()}
+        return v
+
+    def pick(d, *keys):
+        return {k: short(d[k]) for k in keys if k in d}
+
+    out = {k: v for k, v in line.items() if k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                                                  "higher_is_better", "scaling", "vs_baseline", "dtype", "data",
+                                                  "config", "e2e", "gpu_launches", "clocks", "batched_over_plain",
+                                                  "cpu_baseline")}  # fmt: skip
+    for key, keys in (("plain", ("value", "ms_per_step", "bit_identical_to_batched")),
+                      ("plain_reference_calls", ("value", "ms_per_step")), ("unfused", ("value",)),
+                      ("parity", ("frames_checked", "bit_exact")), ("decode", ("fer",)),
+                      ("roofline", ("kernel", "bound", "achieved", "peak", "unit", "frac", "launch_ms"))):  # fmt: skip
+        if key in line:
+            out[key] = pick(line[key], *keys)
+    if "e2e" in out:
+        out["e2e"] = {k: short(v) for k, v in out["e2e"].items() if not isinstance(v, (str, dict)) or k == "unit"}
+        out["e2e"]["value"] = line["e2e"]["value"]
+    c = line.get("configs", {})
+    configs = {k: {"error": v["error"][:80]} for k, v in c.items() if "error" in v}
+    for key in ("3", "1"):
+        if "value" in c.get(key, {}):
+            configs[key] = {"gbps": short(c[key]["value"]), "e2e_gbps": short(c[key]["e2e"]["value"])}
+    for key in ("2", "2_mpoint"):
+        if "results" in c.get(key, {}):
+            configs[key] = {f"{k}_us": short(r["us"]) for k, r in c[key]["results"].items()}
+    if "min_sum" in c.get("reference_ldpc_benchmark", {}):
+        configs["reference_ldpc_benchmark"] = {f"{k}_ms": short(c["reference_ldpc_benchmark"][k]["ms"])
+                                               for k in ("min_sum", "sum_product")}  # fmt: skip
+    for key, field in (("host_overhead", None), ("f1_montecarlo", "blocks_per_s")):
+        if "results" in c.get(key, {}):
+            configs[key] = {k: short(r[field] if field else r) for k, r in c[key]["results"].items()}
+    if "saturation" in c.get("5", {}):
+        configs["5"] = {"saturation_gbps": short(c["5"]["saturation"]["gbps"]),
+                        "p99_ms": {k: short(v["p99_ms"]) for k, v in c["5"]["latency_vs_load"].items()},
+                        "feed_p99_ms_at_70pct": {k: short(v["p99_ms_at_70pct"]) for k, v in c["5"].get("feed", {}).items()
+                                                 if isinstance(v, dict)}}  # fmt: skip
+    if configs:
+        out["configs"] = configs
+    out["details"] = "stderr"
+    return out
+
+
 def main() -> None:
     args = parse()
     if args.impl == "reference":
@@ -1292,6 +1345,9 @@ def main() -> None:
                 except Exception as exc:  # report it and keep the headline line
                     configs[key] = {"error": f"{type(exc).__name__}: {exc}"}
             line["configs"] = configs
+        if args.workload == "mixed":
+            print("details: " + json.dumps(line), file=sys.stderr, flush=True)
+            line = short_line(line)
         print(json.dumps(line), flush=True)
     dist.close()
 
